@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1004,8 +1005,9 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
 // Autotuner of the tile shapes: the first gradient solve of a problem shape
 // on a device times each candidate shape on the solve's own geometry (see
 // solve_device_on's tuning mode) and keeps the fastest for later solves of
-// that shape.  Solves of fewer than AUTOTUNE_MIN_VOXELS voxels, greedy solves
-// and solves with shapes set in the environment take the fixed shapes.
+// that shape.  Solves of fewer than AUTOTUNE_MIN_VOXELS voxels and greedy
+// solves take the default x-y shape at the wave-filled depth; shapes set in
+// the environment come first.
 // ---------------------------------------------------------------------------
 struct TuneKey {
     int device;
@@ -1030,25 +1032,57 @@ bool autotune_enabled() {
     return g_autotune != 0;
 }
 
-// Planes per z tile that fill the waves of a persistent grid of `slots`
-// resident blocks.  The launch is modelled as ceil(tiles / slots) waves of
-// bz + 6 plane-times (a tile forms bz + 4 planes, plus its fixed cost), with
-// tiles(bz) = sum over volumes of (x-y tiles) x ceil(nz / bz); the cheapest
-// bz in [12, 64] wins, the larger one on ties.  At 256^3 with 32 x 16 tiles
-// and 296 slots this gives 29 planes (1152 tiles, 3.9 waves) where 32
-// planes leave the fourth wave less than half full (1024 tiles, 3.5 waves).
-int wave_filled_bz(const std::vector<Geom> &geo, int tile_x, int slots) {
+// Time, in plane-times, of one persistent launch over tiles of bz planes on
+// `slots` resident blocks: the tile queue played through, one layer of
+// tiles (a volume's tiles with the same z range, all equally long) at a
+// time.  A tile of n planes forms n + 4 and costs about two more planes.
+long long queue_time(const std::vector<Geom> &geo, int tile_x, int slots, int bz, long long limit) {
+    struct Free {
+        long long at;
+        long long count;
+    };
+    std::vector<Free> free = {{0, slots}};  // slots by the time they fall free, earliest first
+    long long end = 0;
+    for (const Geom &g : geo) {
+        const long long xy = (long long) ((g.nx + tile_x - 1) / tile_x) * ((g.ny + TT_Y - 1) / TT_Y);
+        for (int z = 0; z < g.nz; z += bz) {
+            const long long len = std::min(bz, g.nz - z) + 6;
+            for (long long left = xy; left > 0;) {
+                const Free f = free.front();
+                const long long n = std::min(left, f.count);
+                left -= n;
+                if (n == f.count) free.erase(free.begin());
+                else free.front().count -= n;
+                const Free done = {f.at + len, n};
+                auto it = free.begin();
+                while (it != free.end() && it->at < done.at) ++it;
+                if (it != free.end() && it->at == done.at) it->count += n;
+                else free.insert(it, done);
+                end = std::max(end, done.at);
+            }
+            if (end >= limit) return end;
+        }
+    }
+    return end;
+}
+
+// Planes per z tile, in [lo, 32], that fill the waves of a persistent grid of
+// `slots` resident blocks: the depth of the shortest launch in queue_time's
+// model, the larger one on ties.  (Deeper tiles cost more than they save: the
+// last ones run alone.  Greedy trial at 256^3: 0.282 ms at 58 planes, 0.274
+// at 32.)  At 256^3 with 32 x 16 tiles and 296 slots this gives 29 planes
+// (1152 tiles, 3.9 waves; 32 planes give 1024 tiles, 3.5 waves).  A
+// volume that does not fill the slots at 32 planes takes thin tiles: a
+// plane costs a block 1.7-2.1 us whether or not its SM has other work, so
+// 40^3 in FP64 is better off as 120 tiles of 6 planes than as 12 of 36
+// (100 iterations: 16.4 -> 4.1 ms).
+int wave_filled_bz(const std::vector<Geom> &geo, int tile_x, int slots, int lo) {
     int mz = 0;
     for (const Geom &g : geo) mz = std::max(mz, g.nz);
     int best = std::min(mz, 32);
-    double best_t = DBL_MAX;
-    for (int bz = std::min(64, mz); bz >= 12; --bz) {
-        long long tiles = 0;
-        for (const Geom &g : geo) {
-            const int b = std::min(bz, g.nz);
-            tiles += (long long) ((g.nx + tile_x - 1) / tile_x) * ((g.ny + TT_Y - 1) / TT_Y) * ((g.nz + b - 1) / b);
-        }
-        const double t = (double) ((tiles + slots - 1) / slots) * (bz + 6);
+    long long best_t = LLONG_MAX;
+    for (int bz = std::min(32, mz); bz >= std::min(lo, mz); --bz) {
+        const long long t = queue_time(geo, tile_x, slots, bz, best_t);
         if (t < best_t) {
             best_t = t;
             best = bz;
@@ -1080,10 +1114,15 @@ template <typename T>
 int choose_config(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols, const dtb_params &p,
                   int precision, TileConfig *out) {
     TileConfig c;
-    if (env_config(sizeof(T), &c) || algorithm != DTB_ALGORITHM_GRADIENT || !autotune_enabled()) {
+    if (env_config(sizeof(T), &c)) {
         *out = c;
         return DTB_OK;
     }
+    std::vector<Geom> geo;
+    for (const DevVol<T> &v : vols) geo.push_back(v.g);
+    const bool gradient = algorithm == DTB_ALGORITHM_GRADIENT;
+    const int slots =
+        std::max(1, gradient ? trial_tma_blocks_per_sm<T>(32, 16) : greedy_tma_blocks_per_sm<T>()) * num_sms();
     TuneKey key{e->device, sizeof(T), (int) vols.size(), 0, 0, 0, 0};
     for (const DevVol<T> &v : vols) {
         key.voxels += (long long) v.g.nx * v.g.ny * v.g.nz;
@@ -1091,7 +1130,8 @@ int choose_config(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols, 
         key.my = std::max(key.my, v.g.ny);
         key.mz = std::max(key.mz, v.g.nz);
     }
-    if (key.voxels < AUTOTUNE_MIN_VOXELS) {
+    if (!gradient || key.voxels < AUTOTUNE_MIN_VOXELS || !autotune_enabled()) {
+        c.bz = wave_filled_bz(geo, 32, slots, 2);
         *out = c;
         return DTB_OK;
     }
@@ -1103,10 +1143,7 @@ int choose_config(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols, 
     NvtxRange range("dtb autotune");
     TileConfig best = c;
     float best_ms = FLT_MAX;
-    std::vector<Geom> geo;
-    for (const DevVol<T> &v : vols) geo.push_back(v.g);
-    const int slots = std::max(1, trial_tma_blocks_per_sm<T>(32, 16)) * num_sms();
-    for (const TileConfig &cand : tile_candidates(sizeof(T), wave_filled_bz(geo, 32, slots))) {
+    for (const TileConfig &cand : tile_candidates(sizeof(T), wave_filled_bz(geo, 32, slots, 12))) {
         float ms = FLT_MAX;
         const int rc = solve_device_on<T>(e, algorithm, vols, p, nullptr, precision, &cand, &ms);
         if (rc != DTB_OK) return rc;

@@ -430,3 +430,19 @@ def test_batched_inplace_equals_copying():
         assert sa["iterations"] == sb["iterations"]
     with pytest.raises(ValueError):
         dt.solve_batched([(vols[0][0], vols[0][1], np.zeros((3, 10, 12, 9), np.float32))], inplace=True)
+
+
+@pytest.mark.parametrize("algorithm", ["gradient", "greedy"])
+@pytest.mark.parametrize("shape", [(3, 20, 33), (40, 40, 40), (37, 18, 70)])
+def test_thin_tiles_equal_deep_tiles(monkeypatch, algorithm, shape):
+    """The z depth a small solve picks by itself (thin tiles that fill the
+    device) gives the FP64 field of 32-plane tiles."""
+    rng = np.random.default_rng(5)
+    Jt = np.ascontiguousarray(1.0 + 0.1 * rng.standard_normal(shape))
+    mask = np.ascontiguousarray(rng.random(shape) < 0.5)
+    thin, st = dt.solve(Jt, mask, algorithm=algorithm, precision="fp64", it_max=12)
+    assert dt.tile_config()["bz"] < min(shape[0], 32) or shape[0] == 3
+    monkeypatch.setenv("DISPTOOLS_B200_BZ", "32")
+    deep, sd = dt.solve(Jt, mask, algorithm=algorithm, precision="fp64", it_max=12)
+    assert dt.tile_config()["bz"] == 32 and st["iterations"] == sd["iterations"]
+    np.testing.assert_array_equal(thin, deep)
