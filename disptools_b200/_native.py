@@ -155,6 +155,8 @@ lib.dtb_log_jacobian_accumulate_device.argtypes = [_I, _I, _SZ, _D, _P, _P, _P]
 lib.dtb_log_jacobian_accumulate_device.restype = _I
 lib.dtb_exp_mean_device.argtypes = [_I, _SZ, _D, _P, _P, _P]
 lib.dtb_exp_mean_device.restype = _I
+lib.dtb_log_jacobian_field_device.argtypes = [_I, _SZ, _SZ, _SZ, _D, _D, _D, _P, _D, _I, _I, _D, _P, _P]
+lib.dtb_log_jacobian_field_device.restype = _I
 lib.volume_matching_3d.argtypes = [_SZ, _SZ, _SZ, _D, _D, _D, _P, _P] + [_D] * 11 + [C.c_bool, _SZ, _P]
 lib.volume_matching_3d.restype = None
 lib.dtb_volume_matching.argtypes = [_SZ, _SZ, _SZ, _D, _D, _D, _P, _P, C.POINTER(Params), _P,
@@ -200,7 +202,7 @@ EXPORTED = [
     "dtb_smooth_recursive_device", "dtb_resample_device",
     "dtb_write_rvf", "dtb_read_rvf_header", "dtb_read_rvf", "dtb_write_vtk", "dtb_read_vtk_header",
     "dtb_read_vtk", "dtb_volume_change_device", "dtb_log_jacobian_accumulate_device",
-    "dtb_exp_mean_device", "volume_matching_3d", "dtb_volume_matching", "dtb_volume_matching_device",
+    "dtb_exp_mean_device", "dtb_log_jacobian_field_device", "volume_matching_3d", "dtb_volume_matching", "dtb_volume_matching_device",
     "dtb_set_verbose",
     "dtb_set_device_memory_limit", "dtb_test_drop_tma_load",
 ]

@@ -39,7 +39,7 @@ UNITS = [
     ("dt_maps.cu", []),
     ("dt_matching.cu", ["-fmad=false"]),
 ]
-HEADERS = ["dt_internal.h", "dt_kernels.cuh", "dt_kernels_tma.cuh", "dt_tma.cuh"]
+HEADERS = ["dt_internal.h", "dt_jacobian.cuh", "dt_kernels.cuh", "dt_kernels_tma.cuh", "dt_tma.cuh"]
 
 
 def _nvcc() -> str:

@@ -1415,13 +1415,26 @@ extern "C" void generate_displacement_greedy_cuda(
 // ---------------------------------------------------------------------------
 namespace {
 
+// FP64 volumes below this many voxels take the element-wise Jacobian kernel
+// and the plain-load gather whatever their layout.  The TMA kernels run one
+// block of 8 warps per SM in FP64, the element-wise one 16 warps: map of
+// 128^3 63.8 us by TMA, 55.9 element-wise (129 x 127 x 125); 180 x 216 x 180
+// 139 and 132; 192 x 224 x 192 148 and 149.  Adjoint of 160^3 391 us by TMA and
+// 272 without, 180 x 216 x 180 434 and 412, 192 x 224 x 192 454 and 493.
+constexpr long long FP64_ELEMENTWISE_VOXELS = 7500000;
+
+template <typename T>
+bool tma_stencil_pays(const Geom &g) {
+    return sizeof(T) == 4 || (long long) g.nx * g.ny * g.nz >= FP64_ELEMENTWISE_VOXELS;
+}
+
 template <typename T>
 int jacobian_device_impl(const Geom &g, const T *field, T *J, cudaStream_t s) {
     // TMA kernel: fourth order, rows a multiple of 16 bytes long, a 16-byte
     // aligned field and pair-aligned J.  It takes its tensor map as a kernel
     // parameter and needs no device memory of its own: no lock, no wait.
-    if (g.order == 4 && (g.ys * (long long) sizeof(T)) % 16 == 0 && reinterpret_cast<uintptr_t>(field) % 16 == 0 &&
-        reinterpret_cast<uintptr_t>(J) % (2 * sizeof(T)) == 0) {
+    if (tma_stencil_pays<T>(g) && g.order == 4 && (g.ys * (long long) sizeof(T)) % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(field) % 16 == 0 && reinterpret_cast<uintptr_t>(J) % (2 * sizeof(T)) == 0) {
         CUtensorMap tm;
         const CUtensorMapDataType ft = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
         if (encode_map(&tm, ft, sizeof(T), field, g, 3, 32 + 2 * 4, TT_Y + 2 * 2)) {
@@ -1429,34 +1442,25 @@ int jacobian_device_impl(const Geom &g, const T *field, T *J, cudaStream_t s) {
             return DTB_OK;
         }
     }
-    // Other layouts and order 2: the plain-load kernel, with its descriptor
-    // in the shared workspace.
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    const int bz = bz_for(g.nz, 32);
-    const int ntiles = ((g.nx + BX - 1) / BX) * ((g.ny + BY - 1) / BY) * ((g.nz + bz - 1) / bz);
-    char *base = nullptr;
-    int rc = workspace(1024 + sizeof(VolumeDesc<T>) + (size_t) ntiles * sizeof(int), &base);
-    if (rc != DTB_OK) return rc;
-    Carve cv{base};
-    VolumeDesc<T> *d_desc = cv.take<VolumeDesc<T>>(1);
-    int *d_tv = cv.take<int>(ntiles);
-    VolumeDesc<T> d;
-    std::memset(&d, 0, sizeof d);
-    d.g = g;
-    d.field[0] = const_cast<T *>(field);
-    d.jout = J;
-    d.tiles_x = (g.nx + BX - 1) / BX;
-    d.tiles_y = (g.ny + BY - 1) / BY;
-    d.tiles_z = (g.nz + bz - 1) / bz;
-    d.tile_begin = 0;
-    d.ntiles = ntiles;
-    d.bz = bz;
-    DTB_CUDA(cudaMemcpyAsync(d_desc, &d, sizeof d, cudaMemcpyHostToDevice, s));
-    DTB_CUDA(cudaMemsetAsync(d_tv, 0, (size_t) ntiles * sizeof(int), s));
-    DTB_CUDA(launch_jacobian<T>(d_desc, d_tv, ntiles, ntiles, s));
-    // The descriptor lives in the shared workspace: finish before releasing it.
-    DTB_CUDA(cudaStreamSynchronize(s));
+    // Other layouts and order 2: the element-wise kernel.  It takes its
+    // geometry as a parameter too: no lock, no wait.
+    DTB_CUDA(launch_jacobian_any<T>(field, g, J, num_sms(), s));
     return DTB_OK;
+}
+
+// Whether the adjoint streams its weights by TMA (k_gather_tma) or reads them
+// by plain loads (k_adjoint_gather), by the voxel counts where the two cross:
+// rows a multiple of 16 bytes long, FP32 100^3 64.5 us by TMA and 62.6 plain,
+// 128^3 85 and 110, 160^3 152 and 182; FP64 see above.  Odd widths (weights
+// padded for TMA, their stores and the gradient's unpaired) FP32 129 x 127 x
+// 125 97 and 93, 160 x 161 x 159 170 and 166, 181 x 217 x 181 252 and 262;
+// FP64 334 and 254, 474 and 400, 255 x 255 x 257 1229 and 995.
+template <typename T>
+bool adjoint_streams_weights(const Geom &g) {
+    if (g.order != 4) return false;
+    const long long n = (long long) g.nx * g.ny * g.nz;
+    if ((g.ys * (long long) sizeof(T)) % 16 == 0) return n >= (sizeof(T) == 4 ? 1ll << 20 : FP64_ELEMENTWISE_VOXELS);
+    return sizeof(T) == 4 && n >= 6000000;
 }
 
 // The adjoint's path: the weight pass and gather by default, the fused TMA
@@ -1482,11 +1486,20 @@ int adjoint_device_impl(const Geom &g, const T *field, const T *gJ, T *gout, cud
     }
     std::lock_guard<std::mutex> lock(g_ws_mutex);
     // Weights W[9][wn] in the adjoint's own buffer, each component 256-byte
-    // aligned.  Calls are ordered on the device, not on the host: this
-    // call's stream waits for the previous call's gather (any stream) before
-    // it overwrites W.  Growing the buffer frees the old one, which waits
-    // for the device.
-    const long long wn = ((long long) g.cs + 63) / 64 * 64;
+    // aligned and, where the gather streams them by TMA, the rows padded to 16
+    // bytes.  Calls are ordered on the device, not on the host: this call's
+    // stream waits for the previous call's gather (any stream) before it
+    // overwrites W.  Growing the buffer frees the old one, which waits for the
+    // device.
+    const bool streams = adjoint_streams_weights<T>(g);
+    Geom gw = g;
+    if (streams) {
+        const long long v = 16 / (long long) sizeof(T);
+        gw.ys = (g.nx + v - 1) / v * v;
+        gw.zs = gw.ys * g.ny;
+        gw.cs = gw.zs * g.nz;
+    }
+    const long long wn = (gw.cs + 63) / 64 * 64;
     char *base = nullptr;
     int rc = grow(g_adj, 9 * (size_t) wn * sizeof(T) + 256, &base);
     if (rc != DTB_OK) return rc;
@@ -1496,28 +1509,25 @@ int adjoint_device_impl(const Geom &g, const T *field, const T *gJ, T *gout, cud
     if (!g_adj_done[dev]) DTB_CUDA(cudaEventCreateWithFlags(&g_adj_done[dev], cudaEventDisableTiming));
     DTB_CUDA(cudaStreamWaitEvent(s, g_adj_done[dev], 0));
     T *W = reinterpret_cast<T *>(base);
-    // The weight pass on the TMA stencil kernel when the layout allows it
-    // (as for the Jacobian map), else on the plain-load kernel.  The gather
-    // pass streams W by TMA after a TMA weight pass (W then has rows a
-    // multiple of 16 bytes long) into a pair-aligned gradient.
-    bool w_done = false;
+    // The weight pass on the TMA stencil kernel when the field's layout
+    // allows it (as for the Jacobian map), else on the element-wise kernel.
     const CUtensorMapDataType ft = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
-    if (g.order == 4 && (g.ys * (long long) sizeof(T)) % 16 == 0 && reinterpret_cast<uintptr_t>(field) % 16 == 0 &&
-        reinterpret_cast<uintptr_t>(gJ) % (2 * sizeof(T)) == 0) {
-        CUtensorMap tm;
-        if (encode_map(&tm, ft, sizeof(T), field, g, 3, 32 + 2 * 4, TT_Y + 2 * 2)) {
-            DTB_CUDA(launch_jacobian_tma<T>(tm, g, nullptr, g.ys, g.zs, num_sms(), s, gJ, W, wn));
-            w_done = true;
-        }
-    }
-    CUtensorMap tw[3];
-    if (w_done && reinterpret_cast<uintptr_t>(gout) % (2 * sizeof(T)) == 0 &&
-        encode_weights_map(&tw[0], ft, sizeof(T), W, g, wn, 32 + 2 * 4, TT_Y) &&
-        encode_weights_map(&tw[1], ft, sizeof(T), W, g, wn, 32, TT_Y + 2 * 2) &&
-        encode_weights_map(&tw[2], ft, sizeof(T), W, g, wn, 32, TT_Y))
-        DTB_CUDA(launch_gather_tma<T>(tw[0], tw[1], tw[2], g, gout, num_sms(), s));
+    CUtensorMap tm, tw[3];
+    if (tma_stencil_pays<T>(g) && g.order == 4 && (g.ys * (long long) sizeof(T)) % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(field) % 16 == 0 && reinterpret_cast<uintptr_t>(gJ) % (2 * sizeof(T)) == 0 &&
+        encode_map(&tm, ft, sizeof(T), field, g, 3, 32 + 2 * 4, TT_Y + 2 * 2))
+        DTB_CUDA(launch_jacobian_tma<T>(tm, g, nullptr, g.ys, g.zs, num_sms(), s, gJ, W, wn));
     else
-        DTB_CUDA(launch_adjoint<T>(g, field, gJ, W, wn, gout, w_done, s));
+        DTB_CUDA(launch_weights_any<T>(field, g, gJ, W, wn, gw.ys, gw.zs, num_sms(), s));
+    if (streams) {
+        if (!(encode_weights_map(&tw[0], ft, sizeof(T), W, gw, wn, 32 + 2 * 4, TT_Y) &&
+              encode_weights_map(&tw[1], ft, sizeof(T), W, gw, wn, 32, TT_Y + 2 * 2) &&
+              encode_weights_map(&tw[2], ft, sizeof(T), W, gw, wn, 32, TT_Y)))
+            DTB_FAIL(DTB_ERR_CUDA, "cannot encode the TMA descriptors (cuTensorMapEncodeTiled)");
+        DTB_CUDA(launch_gather_tma<T>(tw[0], tw[1], tw[2], g, gout, num_sms(), s));
+    } else {
+        DTB_CUDA(launch_adjoint_gather<T>(g, W, wn, gout, s));
+    }
     DTB_CUDA(cudaEventRecord(g_adj_done[dev], s));
     return DTB_OK;
 }
@@ -1537,6 +1547,25 @@ extern "C" int dtb_jacobian_device(int precision, int order, size_t nx, size_t n
     if (precision == DTB_PRECISION_MIXED)
         return jacobian_device_impl<float>(g, static_cast<const float *>(field), static_cast<float *>(J), s);
     DTB_FAIL(DTB_ERR_ARGUMENT, "invalid precision");
+}
+
+extern "C" int dtb_log_jacobian_field_device(int precision, size_t nx, size_t ny, size_t nz, double dx, double dy,
+                                             double dz, const void *field, double epsilon, int first, int last,
+                                             double scale, double *acc, void *stream) {
+    disptools_clear_error();
+    if (!valid_dims(nx, ny, nz)) DTB_FAIL(DTB_ERR_ARGUMENT, "every axis needs at least 3 voxels");
+    if (!field || !acc) DTB_FAIL(DTB_ERR_ARGUMENT, "null array");
+    const Geom g = make_geom(nx, ny, nz, dx, dy, dz, 4);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (precision == DTB_PRECISION_FP64)
+        DTB_CUDA(launch_log_jacobian<double>(static_cast<const double *>(field), g, acc, epsilon, first != 0, last != 0,
+                                             scale, num_sms(), s));
+    else if (precision == DTB_PRECISION_MIXED)
+        DTB_CUDA(launch_log_jacobian<float>(static_cast<const float *>(field), g, acc, epsilon, first != 0, last != 0,
+                                            scale, num_sms(), s));
+    else
+        DTB_FAIL(DTB_ERR_ARGUMENT, "invalid precision");
+    return DTB_OK;
 }
 
 extern "C" int dtb_jacobian_adjoint_device(int precision, int order, size_t nx, size_t ny, size_t nz, double dx,

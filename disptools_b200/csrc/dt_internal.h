@@ -11,11 +11,10 @@
 
 namespace dtb {
 
-// Thread-block shape of every stencil kernel: BX threads along x (one warp,
-// coalesced rows), BY along y; each block marches a z-range of one tile.
+// Tile of the element-wise Jacobian kernel and of the no-allocation entry
+// point's volume limit: BX voxels along x (one warp, coalesced rows), BY along y.
 constexpr int BX = 32;
 constexpr int BY = 8;
-constexpr int NT = BX * BY;
 // Tile height of the TMA kernels of the gradient method (two rows per thread).
 constexpr int TT_Y = 2 * BY;
 
@@ -98,7 +97,6 @@ struct VolumeDesc {
     const T *Jt;             // target Jacobian
     const uint8_t *mask;     // body mask
     T *v[2];                 // greedy: error maps
-    T *jout;                 // jacobian-only launches: output map
     T *ep[2];                // gradient method: regularised error e' of field[i]
     // TMA descriptors (device memory) of field[0..1], grad, ep[0..1] or
     // v[0..1] (three-plane boxes), Jt, mask
@@ -123,18 +121,9 @@ struct VolumeDesc {
     unsigned wait_limit;
 };
 
-// Dynamic shared memory of the Jacobian map kernel (bytes): a five-plane ring.
-template <typename T> constexpr int jacobian_smem_bytes() {
-    return 5 * 3 * (BY + 4) * (BX + 4) * (int) sizeof(T);
-}
-
 // Launch wrappers, instantiated for float and double in dt_kernels_*.cu.
 // `work_flag` (may be null) is set to 1 by a launch that did work for at
 // least one volume (profiling separates real launches from no-op ones).
-// Jacobian map of field[0] of each volume into its jout (tiles BX x BY).
-template <typename T>
-cudaError_t launch_jacobian(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
-                            cudaStream_t s);
 // TMA kernels of the gradient method; tiles are tile_x (64 or 32) by TT_Y
 // voxels; threads_y rows of threads (8 or 16).  `pf` > 0 prefetches into L2
 // the boxes of the plane pf iterations ahead of each load.
@@ -188,11 +177,22 @@ cudaError_t launch_gather_tma(const CUtensorMap &tm_wx, const CUtensorMap &tm_wy
 template <typename T>
 cudaError_t launch_adjoint_tma(const CUtensorMap &tm_u, const Geom &g, const T *gJ, T *gout, int num_sms,
                                cudaStream_t s);
-// Adjoint of the Jacobian stencil: the weight pass (unless w_done: W already
-// holds the weights) and the gather pass; W is [9][N] with component stride wn.
+// Gather pass of the adjoint by plain loads, either order: W is dense, [9][N]
+// with component stride wn.
 template <typename T>
-cudaError_t launch_adjoint(const Geom &g, const T *field, const T *gJ, T *W, long long wn, T *gout, bool w_done,
-                           cudaStream_t s);
+cudaError_t launch_adjoint_gather(const Geom &g, const T *W, long long wn, T *gout, cudaStream_t s);
+// The Jacobian stencil of one field in any row layout and order: the map, the
+// adjoint's weights (component stride wn, row and plane strides wys, wzs), and
+// the log of the FP64 map, clamped from below at eps, added to acc (`first`:
+// stored in it; `last`: exp(scale * sum) stored in it).
+template <typename T>
+cudaError_t launch_jacobian_any(const T *field, const Geom &g, T *J, int num_sms, cudaStream_t s);
+template <typename T>
+cudaError_t launch_weights_any(const T *field, const Geom &g, const T *gJ, T *W, long long wn, long long wys,
+                               long long wzs, int num_sms, cudaStream_t s);
+template <typename TI>
+cudaError_t launch_log_jacobian(const TI *field, const Geom &g, double *acc, double eps, bool first, bool last,
+                                double scale, int num_sms, cudaStream_t s);
 template <typename T>
 cudaError_t launch_convert(const void *src, int src_is_double, T *dst, long long n, cudaStream_t s);
 template <typename T>

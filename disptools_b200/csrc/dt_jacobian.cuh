@@ -1,0 +1,324 @@
+// Jacobian stencil of one field in any row layout (sm_100a): the map, the
+// adjoint's weights, or the log of the map added to a running sum.
+//
+// The TMA kernels need rows a multiple of 16 bytes long.  Every other layout
+// (odd widths, a base off a 16-byte boundary), second order, and FP64
+// arithmetic on float fields come here.
+//
+// A block of 32 x 8 threads, one voxel each, marches a 32 x 8 tile through
+// bz planes.  Boxes of the tile with two voxels of halo on each x-y side and
+// three components arrive element by element with cp.async, JA_D planes
+// ahead, in a ring of JA_NS slots; values outside the volume arrive as
+// zeros.  Each thread keeps its column's values of the planes ze-2 .. ze+2 in
+// registers, so a slot is free once its plane has been the stencil's centre
+// plane, and one block barrier a plane guards everything.  The geometry is a
+// kernel parameter: a launch needs no device memory, no lock and no wait.
+//
+// What bounds it: instruction issue and the latency of a plane's chain, so
+// resident warps: one voxel a thread keeps FP32 at 64 registers (four blocks,
+// 32 warps an SM).  Measured against the plain-load kernel it replaced
+// (256 threads, a 64-bit index per load, scheme by case analysis): see the
+// launch wrapper.
+#pragma once
+
+#include <algorithm>
+#include <climits>
+
+#include "dt_kernels.cuh"
+#include "dt_tma.cuh"
+
+namespace dtb {
+
+constexpr int JA_X = BX, JA_Y = BY, JA_NT = JA_X * JA_Y;
+constexpr int JA_PX = JA_X + 4, JA_PY = JA_Y + 4, JA_ROWS = 3 * JA_PY, JA_PLANE = JA_ROWS * JA_PX;
+constexpr int JA_D = 3, JA_NS = JA_D + 3;
+// Copies: 252 threads take 36 columns of 7 rows at a time.
+constexpr int JA_RG = JA_NT / JA_PX, JA_SWEEPS = (JA_ROWS + JA_RG - 1) / JA_RG;
+
+// Resident blocks per SM: 32 warps at 64 registers (FP32), 16 at 128 (FP64).
+template <typename T>
+__host__ __device__ constexpr int ja_blocks() {
+    return sizeof(T) == 4 ? 4 : 2;
+}
+
+enum JacEpilogue { JAC_MAP = 0, JAC_WEIGHTS = 1, JAC_LOG = 2 };
+
+// Epilogue arguments; arrays of scalars have the field's row and plane
+// strides unless stated.
+template <typename T>
+struct JacOut {
+    T *J = nullptr;          // JAC_MAP
+    const T *gJ = nullptr;   // JAC_WEIGHTS: W[c][a] = gJ cof_ca(I + A) ih_a
+    T *W = nullptr;          //   component stride wn, row and plane strides wys, wzs
+    long long wn = 0, wys = 0, wzs = 0;
+    double *acc = nullptr;   // JAC_LOG: the sum so far (not read by the first)
+    double eps = 0.0, scale = 0.0;
+    int first = 0, last = 0;  // the last writes exp(scale * sum) instead
+};
+
+// Copies BYTES bytes to shared memory, zeros when !ok.
+template <int BYTES>
+__device__ __forceinline__ void cp_async_or_zero(void *dst_smem, const void *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(dst_smem)), "l"(src), "n"(BYTES),
+                 "r"(ok ? BYTES : 0)
+                 : "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// The two central schemes of one axis as one expression of the first and
+// second differences, so that a warp with voxels of both kinds evaluates it
+// once: weights chosen per voxel, and the second difference dropped (not
+// multiplied by zero: it may be infinite) where the scheme is second order.
+// Each rounds as its scheme does: FP32 d1 k1 + d2 k2 fused, or d1 (ih / 2);
+// FP64 ((d1 w1) - d2 / 12) ih half, with w1 = 2/3 and half = 1, or w1 = 1,
+// d2 = 0 and half = 1/2 (exact factors).
+template <typename T>
+struct CentralWeights {
+    T k1[3], k2[3];  // FP32; FP64: k2 = ih
+    T w1, half;      // FP64
+    __device__ __forceinline__ CentralWeights(const T (&ih)[3], bool c4) {
+        w1 = c4 ? FD<T>::two_thirds : T(1);
+        half = c4 ? T(1) : T(.5);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            k1[a] = c4 ? FD<T>::two_thirds * ih[a] : ih[a] * T(.5);
+            k2[a] = sizeof(T) == 4 ? -FD<T>::one_twelfth * ih[a] : ih[a];
+        }
+    }
+    __device__ __forceinline__ T operator()(T d1, T d2, int a) const {
+        if constexpr (sizeof(T) == 4) return __fmaf_rn(d1, k1[a], __fmul_rn(d2, k2[a]));
+        else return (d1 * w1 - d2 * FD<T>::one_twelfth) * k2[a] * half;
+    }
+};
+
+// The stencil matrix of a voxel: `p` its element of the centre plane's box,
+// zq its column's values of planes ze-2 .. ze+2.  A warp is one row of the
+// tile, so `deep` (all its voxels take fourth-order differences) is uniform.
+// Other voxels take fourth-order differences where `c4`, and are second order
+// along every axis elsewhere (schemes_at), one-sided where they lie on a face.
+template <typename TI, typename T>
+__device__ __forceinline__ void stencil_voxel(const TI *p, const TI (&zq)[3][5], int x, int y, int z, const Geom &g,
+                                              const T (&ih)[3], bool deep, bool c4, T (&a)[3][3]) {
+    const CentralWeights<T> w(ih, deep || c4);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const TI *q = p + c * JA_PY * JA_PX;
+        const T xd2 = (T) q[2] - (T) q[-2], yd2 = (T) q[2 * JA_PX] - (T) q[-2 * JA_PX], zd2 = (T) zq[c][4] - (T) zq[c][0];
+        a[c][0] = w((T) q[1] - (T) q[-1], deep || c4 ? xd2 : T(0), 0);
+        a[c][1] = w((T) q[JA_PX] - (T) q[-JA_PX], deep || c4 ? yd2 : T(0), 1);
+        a[c][2] = w((T) zq[c][3] - (T) zq[c][1], deep || c4 ? zd2 : T(0), 2);
+    }
+    if (deep) return;
+    if (x == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const TI *q = p + c * JA_PY * JA_PX;
+            a[c][0] = fd_fwd<T>(q[0], q[1], q[2], ih[0]);
+        }
+    }
+    if (x == g.nx - 1) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const TI *q = p + c * JA_PY * JA_PX;
+            a[c][0] = fd_bwd<T>(q[0], q[-1], q[-2], ih[0]);
+        }
+    }
+    if (y == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const TI *q = p + c * JA_PY * JA_PX;
+            a[c][1] = fd_fwd<T>(q[0], q[JA_PX], q[2 * JA_PX], ih[1]);
+        }
+    }
+    if (y == g.ny - 1) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const TI *q = p + c * JA_PY * JA_PX;
+            a[c][1] = fd_bwd<T>(q[0], q[-JA_PX], q[-2 * JA_PX], ih[1]);
+        }
+    }
+    if (z == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c][2] = fd_fwd<T>(zq[c][2], zq[c][3], zq[c][4], ih[2]);
+    }
+    if (z == g.nz - 1) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c][2] = fd_bwd<T>(zq[c][2], zq[c][1], zq[c][0], ih[2]);
+    }
+}
+
+template <typename TI, typename T, int EPI>
+__global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
+    k_jacobian_async(const TI *__restrict__ field, const Geom g, const JacOut<T> out, int bz) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TI *ring = reinterpret_cast<TI *>(smem_raw);
+    __shared__ long long s_row[JA_ROWS];  // start of each box row in plane 0, -1 outside the volume
+    const int tid = threadIdx.x, tx = tid % JA_X, ty = tid / JA_X;
+    const int tiles_x = (g.nx + JA_X - 1) / JA_X, tiles_y = (g.ny + JA_Y - 1) / JA_Y;
+    const int txy = (int) blockIdx.x / tiles_x;
+    const int x0 = ((int) blockIdx.x - txy * tiles_x) * JA_X, y0 = (txy % tiles_y) * JA_Y, z0 = (txy / tiles_y) * bz;
+    const int z1 = min(z0 + bz, g.nz);
+    if (tid < JA_ROWS) {
+        const int c = tid / JA_PY, gy = y0 - 2 + tid % JA_PY;
+        s_row[tid] = gy >= 0 && gy < g.ny ? c * g.cs + gy * g.ys : -1;
+    }
+    __syncthreads();
+    const int col = tid % JA_PX, rg = tid / JA_PX;
+    const int gx = x0 - 2 + col;
+    const bool copies = tid < JA_RG * JA_PX, col_ok = gx >= 0 && gx < g.nx;
+    // Copies plane zp (tile and halo) into its slot; always one group.
+    auto load_plane = [&](int zp, int slot) {
+        if (copies && zp <= z1 + 1) {
+            TI *dst = ring + slot * JA_PLANE + rg * JA_PX + col;
+            const bool ok = col_ok && zp >= 0 && zp < g.nz;
+            const TI *src = field + (zp * g.zs + gx);
+#pragma unroll
+            for (int k = 0; k < JA_SWEEPS; ++k) {
+                if ((k + 1) * JA_RG > JA_ROWS && rg + k * JA_RG >= JA_ROWS) break;
+                const long long r = s_row[rg + k * JA_RG];
+                const bool in = ok && r >= 0;
+                cp_async_or_zero<(int) sizeof(TI)>(dst + k * JA_RG * JA_PX, in ? src + r : field, in);
+            }
+        }
+        cp_async_commit();
+    };
+    for (int j = 0; j < JA_D; ++j) load_plane(z0 - 2 + j, j);
+
+    const int x = x0 + tx, y = y0 + ty;
+    const bool in_xy = x < g.nx && y < g.ny;
+    const T ih[3] = {(T) g.ih[0], (T) g.ih[1], (T) g.ih[2]};
+    const bool row_in = y >= 2 && y <= g.ny - 3 && g.order == 4;
+    const bool tile_in = row_in && x0 >= 2 && x0 + JA_X - 1 <= g.nx - 3;
+    const bool voxel_in = row_in && x >= 2 && x <= g.nx - 3;
+    const int own = (ty + 2) * JA_PX + tx + 2;
+    TI zq[3][5];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 5; ++k) zq[c][k] = TI(0);
+    long long off = (z0 - 4) * g.zs + y * g.ys + x;  // of the thread's voxel in plane ze
+    int slot = 0;                                    // of plane q
+    for (int q = z0 - 2; q <= z1 + 1; ++q, off += g.zs) {
+        cp_async_wait_group<JA_D - 1>();
+        __syncthreads();
+        // The slot of plane q + D held plane q - 3, the last centre plane.
+        load_plane(q + JA_D, slot + JA_D < JA_NS ? slot + JA_D : slot + JA_D - JA_NS);
+        const TI *pl = ring + slot * JA_PLANE + own;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) zq[c][k] = zq[c][k + 1];
+            zq[c][4] = pl[c * JA_PY * JA_PX];
+        }
+        const int ze = q - 2;
+        const int se = slot >= 2 ? slot - 2 : slot - 2 + JA_NS;
+        slot = slot + 1 < JA_NS ? slot + 1 : 0;
+        if (ze < z0 || !in_xy) continue;
+        const bool plane_in = ze >= 2 && ze <= g.nz - 3;
+        T a[3][3];
+        stencil_voxel<TI, T>(ring + se * JA_PLANE + own, zq, x, y, ze, g, ih, tile_in && plane_in,
+                             voxel_in && plane_in, a);
+        if constexpr (EPI == JAC_MAP) {
+            out.J[off] = det_i_plus<T>(a);
+        } else if constexpr (EPI == JAC_LOG) {
+            double j = (double) det_i_plus<T>(a);
+            j = j < out.eps ? out.eps : j;
+            double s = log(j);
+            if (!out.first) s = out.acc[off] + s;
+            out.acc[off] = out.last ? exp(out.scale * s) : s;
+        } else {
+            const T w = out.gJ[off];
+            T *W = out.W + (ze * out.wzs + y * out.wys + x);
+            a[0][0] += T(1);
+            a[1][1] += T(1);
+            a[2][2] += T(1);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int r0 = c == 0 ? 1 : 0, r1 = c == 2 ? 1 : 2;
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const int c0 = b == 0 ? 1 : 0, c1 = b == 2 ? 1 : 2;
+                    const T minor = a[r0][c0] * a[r1][c1] - a[r0][c1] * a[r1][c0];
+                    const T cof = ((c + b) & 1) ? -minor : minor;
+                    W[(c * 3 + b) * out.wn] = w * cof * ih[b];
+                }
+            }
+        }
+    }
+    cp_async_wait_all();
+}
+
+// Planes per block: thin tiles where the volume does not fill the device.  A
+// block of bz planes takes bz + 4 plane-times and about two more to start;
+// below one wave of blocks the launch lasts that long, above it the blocks
+// backfill and half a block is left over at the end.
+inline int jacobian_depth(const Geom &g, int slots) {
+    const double cols = (double) ((g.nx + JA_X - 1) / JA_X) * ((g.ny + JA_Y - 1) / JA_Y);
+    int best = 1;
+    double best_t = 1e300;
+    for (int bz = std::min(g.nz, 32); bz >= 2; --bz) {
+        const double waves = cols * ((g.nz + bz - 1) / bz) / slots;
+        const double t = (bz + 6) * (waves <= 1.0 ? 1.0 : waves + 0.5);
+        if (t < best_t) {
+            best_t = t;
+            best = bz;
+        }
+    }
+    return best;
+}
+
+template <typename TI, typename T, int EPI>
+cudaError_t launch_jacobian_async(const TI *field, const Geom &g, const JacOut<T> &out, int num_sms, cudaStream_t s) {
+    constexpr int smem = JA_NS * JA_PLANE * (int) sizeof(TI);
+    static std::atomic<unsigned long long> devs{0};
+    const cudaError_t attr = opt_in_smem(k_jacobian_async<TI, T, EPI>, smem, devs);
+    if (attr != cudaSuccess) return attr;
+    const int bz = jacobian_depth(g, ja_blocks<T>() * num_sms);
+    const long long grid =
+        (long long) ((g.nx + JA_X - 1) / JA_X) * ((g.ny + JA_Y - 1) / JA_Y) * ((g.nz + bz - 1) / bz);
+    if (grid > INT_MAX) return cudaErrorInvalidConfiguration;
+    k_jacobian_async<TI, T, EPI><<<(unsigned) grid, JA_NT, smem, s>>>(field, g, out, bz);
+    count_launch();
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_jacobian_any(const T *field, const Geom &g, T *J, int num_sms, cudaStream_t s) {
+    JacOut<T> o;
+    o.J = J;
+    return launch_jacobian_async<T, T, JAC_MAP>(field, g, o, num_sms, s);
+}
+
+template <typename T>
+cudaError_t launch_weights_any(const T *field, const Geom &g, const T *gJ, T *W, long long wn, long long wys,
+                               long long wzs, int num_sms, cudaStream_t s) {
+    JacOut<T> o;
+    o.gJ = gJ;
+    o.W = W;
+    o.wn = wn;
+    o.wys = wys;
+    o.wzs = wzs;
+    return launch_jacobian_async<T, T, JAC_WEIGHTS>(field, g, o, num_sms, s);
+}
+
+template <typename TI>
+cudaError_t launch_log_jacobian(const TI *field, const Geom &g, double *acc, double eps, bool first, bool last,
+                                double scale, int num_sms, cudaStream_t s) {
+    JacOut<double> o;
+    o.acc = acc;
+    o.eps = eps;
+    o.scale = scale;
+    o.first = first;
+    o.last = last;
+    return launch_jacobian_async<TI, double, JAC_LOG>(field, g, o, num_sms, s);
+}
+
+#define DTB_INSTANTIATE_JACOBIAN(T)                                                                            \
+    template cudaError_t launch_jacobian_any<T>(const T *, const Geom &, T *, int, cudaStream_t);              \
+    template cudaError_t launch_weights_any<T>(const T *, const Geom &, const T *, T *, long long, long long,  \
+                                               long long, int, cudaStream_t);
+
+}  // namespace dtb

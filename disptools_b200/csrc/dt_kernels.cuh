@@ -144,42 +144,6 @@ __device__ __forceinline__ int ring_slot(int z, int ns) {
     return s < 0 ? s + ns : s;
 }
 
-// Shared-memory ring of z planes: [NS][3][PY][PX].
-template <typename T, int PX, int PY>
-struct Ring {
-    T *base;
-    __device__ __forceinline__ T &at(int slot, int c, int ly, int lx) const {
-        return base[((slot * 3 + c) * PY + ly) * PX + lx];
-    }
-};
-
-// Derivative of component c along axis `a` with scheme k at ring cell
-// (lx, ly) of plane z (slots of z-2..z+2 in s[0..4]).
-template <typename T, int PX, int PY>
-__device__ __forceinline__ T ring_deriv(const Ring<T, PX, PY> &r, const int s[5], int c, int lx,
-                                        int ly, int a, int k, T ih) {
-    auto val = [&](int o) -> T {
-        if (a == 0) return r.at(s[2], c, ly, lx + o);
-        if (a == 1) return r.at(s[2], c, ly + o, lx);
-        return r.at(s[2 + o], c, ly, lx);
-    };
-    switch (k) {
-    case S_FWD: return fd_fwd<T>(val(0), val(1), val(2), ih);
-    case S_BWD: return fd_bwd<T>(val(0), val(-1), val(-2), ih);
-    case S_C2: return fd_c2<T>(val(1), val(-1), ih);
-    default: return fd_c4<T>(val(1), val(-1), val(2), val(-2), ih);
-    }
-}
-
-template <typename T, int PX, int PY>
-__device__ __forceinline__ void ring_matrix(const Ring<T, PX, PY> &r, const int s[5], int lx, int ly,
-                                            const int k[3], const T ih[3], T a[3][3]) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) a[c][ax] = ring_deriv<T, PX, PY>(r, s, c, lx, ly, ax, k[ax], ih[ax]);
-}
-
 // Per-voxel error of src/headers/error.h:128-142.
 template <typename T>
 __device__ __forceinline__ T voxel_error(T J, T Jt, bool in_mask, T tol) {
@@ -376,115 +340,13 @@ __device__ __forceinline__ T ldcg(const T *p) {
 __device__ __forceinline__ int ldcg_int(const int *p) { return __ldcg(p); }
 
 // ------------------------------------------------------------------------
-// Jacobian map kernel: J = det(I + grad f) of field[0] into jout
-// (src/jacobian.c:113-241), for fields in any row layout.  A block owns a
-// BX x BY tile and marches bz planes with a five-plane shared ring (halo 2).
-// ------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(NT) k_jacobian(const VolumeDesc<T> *__restrict__ vols,
-                                                 const int *__restrict__ tile_vol, int total_tiles) {
-    constexpr int H = 2, PX = BX + 2 * H, PY = BY + 2 * H, NS = 5;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Ring<T, PX, PY> ring{reinterpret_cast<T *>(smem_raw)};
-
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * BX + tx;
-
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-        const VolumeDesc<T> &V = vols[tile_vol[tile]];
-        const Geom g = V.g;
-        const int lt = tile - V.tile_begin;
-        const int txi = lt % V.tiles_x, tyi = (lt / V.tiles_x) % V.tiles_y, tzi = lt / (V.tiles_x * V.tiles_y);
-        const int x0 = txi * BX, y0 = tyi * BY, z0 = tzi * V.bz;
-        const int z1 = min(z0 + V.bz, g.nz);
-        const T *src = V.field[0];
-        const T ih[3] = {(T) g.ih[0], (T) g.ih[1], (T) g.ih[2]};
-
-        // Fill the ring slot of plane zq (tile + halo 2; 0 outside the volume).
-        auto load_plane = [&](int zq) {
-            const int slot = ring_slot(zq, NS);
-            const bool zin = zq >= 0 && zq < g.nz;
-            for (int i = tid; i < 3 * PY * PX; i += NT) {
-                const int c = i / (PY * PX);
-                const int r = i - c * (PY * PX);
-                const int ly = r / PX, lx = r - ly * PX;
-                const int gx = x0 - H + lx, gy = y0 - H + ly;
-                T val = T(0);
-                if (zin && gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny)
-                    val = src[c * g.cs + (long long) zq * g.zs + (long long) gy * g.ys + gx];
-                ring.at(slot, c, ly, lx) = val;
-            }
-        };
-
-        for (int zq = z0 - 2; zq < z0 + 2; ++zq) load_plane(zq);
-
-        const int x = x0 + tx, y = y0 + ty;
-        const bool in_xy = x < g.nx && y < g.ny;
-        for (int z = z0; z < z1; ++z) {
-            load_plane(z + 2);
-            __syncthreads();
-            if (in_xy) {
-                int k[3];
-                schemes_at(x, y, z, g, k);
-                const int s[5] = {ring_slot(z - 2, NS), ring_slot(z - 1, NS), ring_slot(z, NS),
-                                  ring_slot(z + 1, NS), ring_slot(z + 2, NS)};
-                T a[3][3];
-                ring_matrix<T, PX, PY>(ring, s, tx + H, ty + H, k, ih, a);
-                V.jout[(long long) z * g.zs + (long long) y * g.ys + x] = det_i_plus<T>(a);
-            }
-            __syncthreads();
-        }
-    }
-}
-
-// ------------------------------------------------------------------------
 // Exact adjoint of the Jacobian stencil (for autograd).
-// Pass 1: W[c][a](p) = w(p) * cof_ca(I + A(p)) * ih_a, A the stencil matrix.
+// Pass 1 (k_jacobian_tma or k_jacobian_async): W[c][a](p) = w(p) *
+// cof_ca(I + A(p)) * ih_a, A the stencil matrix.
 // Pass 2: grad_c(q) = sum_a sum_t W[c][a](q - t e_a) * kappa(k_a(q - t e_a), t).
-// W is dense, [9][nz][ny][nx] with component stride wn.
+// W is dense, [9][nz][ny][nx] with component stride wn.  Where the caller
+// prefers this gather to k_gather_tma: adjoint_streams_weights in dt_capi.cu.
 // ------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ T gload_deriv(const T *f, long long o, long long s, int k, T ih) {
-    switch (k) {
-    case S_FWD: return fd_fwd<T>(f[o], f[o + s], f[o + 2 * s], ih);
-    case S_BWD: return fd_bwd<T>(f[o], f[o - s], f[o - 2 * s], ih);
-    case S_C2: return fd_c2<T>(f[o + s], f[o - s], ih);
-    default: return fd_c4<T>(f[o + s], f[o - s], f[o + 2 * s], f[o - 2 * s], ih);
-    }
-}
-
-template <typename T>
-__global__ void k_adjoint_w(Geom g, const T *__restrict__ f, const T *__restrict__ gJ, T *__restrict__ W,
-                            long long wn) {
-    const long long N = (long long) g.nx * g.ny * g.nz;
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < N;
-         i += (long long) gridDim.x * blockDim.x) {
-        const int x = (int) (i % g.nx);
-        const int y = (int) ((i / g.nx) % g.ny);
-        const int z = (int) (i / ((long long) g.nx * g.ny));
-        int k[3];
-        schemes_at(x, y, z, g, k);
-        const long long o = (long long) z * g.zs + (long long) y * g.ys + x;
-        const long long st[3] = {1, g.ys, g.zs};
-        T m[3][3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) m[c][a] = gload_deriv<T>(f + c * g.cs, o, st[a], k[a], (T) g.ih[a]) + (c == a ? T(1) : T(0));
-        const T w = gJ[o];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int r0 = c == 0 ? 1 : 0, r1 = c == 2 ? 1 : 2;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const int c0 = a == 0 ? 1 : 0, c1 = a == 2 ? 1 : 2;
-                const T minor = m[r0][c0] * m[r1][c1] - m[r0][c1] * m[r1][c0];
-                const T cof = ((c + a) & 1) ? -minor : minor;
-                W[(c * 3 + a) * wn + i] = w * cof * (T) g.ih[a];
-            }
-        }
-    }
-}
-
 template <typename T>
 __device__ __forceinline__ T kappa(int k, int t) {
     switch (k) {
@@ -619,25 +481,8 @@ inline int elementwise_grid(long long n) {
 }
 
 template <typename T>
-cudaError_t launch_jacobian(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
-                            cudaStream_t s) {
-    constexpr int smem = jacobian_smem_bytes<T>();
-    static std::atomic<unsigned long long> devs{0};
-    const cudaError_t attr = opt_in_smem(k_jacobian<T>, smem, devs);
-    if (attr != cudaSuccess) return attr;
-    k_jacobian<T><<<grid, dim3(BX, BY), smem, s>>>(vols, tile_vol, total_tiles);
-    count_launch();
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_adjoint(const Geom &g, const T *field, const T *gJ, T *W, long long wn, T *gout, bool w_done,
-                           cudaStream_t s) {
+cudaError_t launch_adjoint_gather(const Geom &g, const T *W, long long wn, T *gout, cudaStream_t s) {
     const long long N = (long long) g.nx * g.ny * g.nz;
-    if (!w_done) {
-        k_adjoint_w<T><<<elementwise_grid(N), 256, 0, s>>>(g, field, gJ, W, wn);
-        count_launch();
-    }
     k_adjoint_gather<T><<<elementwise_grid(N), 256, 0, s>>>(g, W, wn, gout);
     count_launch();
     return cudaGetLastError();
@@ -690,9 +535,7 @@ cudaError_t launch_regularise(T *J, long long n, double eps, cudaStream_t s) {
 }
 
 #define DTB_INSTANTIATE(T)                                                                                   \
-    template cudaError_t launch_jacobian<T>(const VolumeDesc<T> *, const int *, int, int, cudaStream_t);     \
-    template cudaError_t launch_adjoint<T>(const Geom &, const T *, const T *, T *, long long, T *, bool,    \
-                                           cudaStream_t);                                                    \
+    template cudaError_t launch_adjoint_gather<T>(const Geom &, const T *, long long, T *, cudaStream_t);    \
     template cudaError_t launch_convert<T>(const void *, int, T *, long long, cudaStream_t);                 \
     template cudaError_t launch_to_double<T>(const T *, double *, long long, cudaStream_t);                  \
     template cudaError_t launch_regularise<T>(T *, long long, double, cudaStream_t);                        \

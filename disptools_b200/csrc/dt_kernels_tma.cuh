@@ -23,6 +23,7 @@
 #pragma once
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <type_traits>
 
@@ -30,6 +31,32 @@
 #include "dt_tma.cuh"
 
 namespace dtb {
+
+// Planes per z tile of a launch that deals `cols` columns of tiles round-robin
+// to `slots` resident blocks.  Where 32-plane tiles fill the device: as many z
+// tiles per column as fit in the waves they need.  Below that, thin tiles: the
+// depth in [2, 32] with the shortest sum of waves, a tile of bz planes taking
+// bz + 4 plane-times and about two more to start (Jacobian map of 64^3 in FP32
+// 18.4 -> 12.2 us, its adjoint 51 -> 26 us, against at least 8 planes a tile).
+inline int wave_depth(int cols, int nz, int slots) {
+    int nzt = (nz + 31) / 32;
+    if ((long long) cols * nzt >= slots) {
+        const int waves = (cols * nzt + slots - 1) / slots;
+        nzt = std::min((nz + 7) / 8, std::max(nzt, waves * slots / cols));
+        return (nz + nzt - 1) / nzt;
+    }
+    int best = 1;
+    long long best_t = LLONG_MAX;
+    for (int bz = std::min(nz, 32); bz >= 2; --bz) {
+        const long long tiles = (long long) cols * ((nz + bz - 1) / bz);
+        const long long t = (tiles + slots - 1) / slots * (bz + 6);
+        if (t < best_t) {
+            best_t = t;
+            best = bz;
+        }
+    }
+    return best;
+}
 
 constexpr int TMA_HX = 4;                  // x halo of the boxes (16-byte aligned start)
 constexpr int TMA_HY = 2;                  // y halo
@@ -2182,14 +2209,11 @@ int jacobian_blocks_v() {
 
 // Jacobian map (or adjoint weights) of the field `tm_u` describes (geometry
 // g, order 4) into jout (strides jys, jzs): tiles of 32 x TT_Y voxels, 16 x 16 threads, as many
-// blocks as fit on the device.  Tiles are dealt round-robin, so the z split
-// is chosen to fill whole waves of the grid: about 32 planes a tile, then as
-// many z tiles per column as fit in that many waves (at least 8 planes a
-// tile, since each tile also loads 4 halo planes).
+// blocks as fit on the device, z split by wave_depth.
 template <typename T, bool ADJ, bool COF>
 cudaError_t launch_jacobian_tma_v(const CUtensorMap &tm_u, const Geom &g, T *jout, long long jys, long long jzs,
                                   int num_sms, cudaStream_t s, const T *gJ, T *W, long long wn) {
-    constexpr int TXW = 32, TYT = 16, BZ = 32;
+    constexpr int TXW = 32, TYT = 16;
     constexpr int smem = JacTmaLayout<T, TXW>::BYTES + 128;
     static std::atomic<unsigned long long> devs{0};
     const cudaError_t attr = opt_in_smem(k_jacobian_tma<T, TXW, TYT, ADJ, COF>, smem, devs);
@@ -2197,10 +2221,7 @@ cudaError_t launch_jacobian_tma_v(const CUtensorMap &tm_u, const Geom &g, T *jou
     const int tiles_x = (g.nx + TXW - 1) / TXW, tiles_y = (g.ny + TT_Y - 1) / TT_Y;
     const int cols = tiles_x * tiles_y;
     const int slots = std::max(1, jacobian_blocks_v<T, TXW, TYT, ADJ, COF>()) * num_sms;  // resident blocks
-    int nzt = (g.nz + BZ - 1) / BZ;                                             // z tiles per column
-    const int waves = (cols * nzt + slots - 1) / slots;
-    nzt = std::min((g.nz + 7) / 8, std::max(nzt, waves * slots / cols));  // at least 8 planes a tile
-    const int bz = (g.nz + nzt - 1) / nzt;
+    const int bz = wave_depth(cols, g.nz, slots);
     const int ntiles = cols * ((g.nz + bz - 1) / bz);
     const int grid = std::min(ntiles, slots);
     k_jacobian_tma<T, TXW, TYT, ADJ, COF><<<grid, dim3(TXW / 2, TYT), smem, s>>>(tm_u, g, jout, jys, jzs, tiles_x,
@@ -2321,6 +2342,8 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, sizeof(T) == 4 ? 3 : 1)
 
         const int x = x0 + 2 * tx;  // this thread's columns: x, x + 1
         const bool pair_in = x + 1 < g.nx;
+        // Stores as pairs where the gradient's rows keep them aligned.
+        const bool pair_st = pair_in && g.ys % 2 == 0 && reinterpret_cast<uintptr_t>(gout) % (2 * sizeof(T)) == 0;
         // Own pair's W[c][z] of planes q-4 .. q (index 2 - t holds plane ze - t).
         P2 wq[RYT][3][5];
 #pragma unroll
@@ -2586,12 +2609,15 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, sizeof(T) == 4 ? 3 : 1)
                 }
                 if (!valid) continue;
                 T *o = gout + (long long) ze * g.zs + (long long) y * g.ys + x;
-                if (pair_in) {
+                if (pair_st) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) st_pair(o + c * g.cs, acc[0][c], acc[1][c]);
                 } else {
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) o[c * g.cs] = acc[0][c];
+                    for (int c = 0; c < 3; ++c) {
+                        o[c * g.cs] = acc[0][c];
+                        if (pair_in) o[c * g.cs + 1] = acc[1][c];
+                    }
                 }
             }
         }
@@ -2642,7 +2668,7 @@ int gather_blocks_v() {
 template <typename T, bool GJ>
 cudaError_t launch_gather_tma_v(const CUtensorMap &tm_wx, const CUtensorMap &tm_wy, const CUtensorMap &tm_wz,
                                 const CUtensorMap &tm_gj, const Geom &g, T *gout, int num_sms, cudaStream_t s) {
-    constexpr int TXW = 32, TYT = 16, BZ = 32;
+    constexpr int TXW = 32, TYT = 16;
     constexpr int smem = GatherTmaLayout<T, TXW, GJ>::BYTES + 128;
     static std::atomic<unsigned long long> devs{0};
     const cudaError_t attr = opt_in_smem(k_gather_tma<T, TXW, TYT, GJ>, smem, devs);
@@ -2650,10 +2676,7 @@ cudaError_t launch_gather_tma_v(const CUtensorMap &tm_wx, const CUtensorMap &tm_
     const int tiles_x = (g.nx + TXW - 1) / TXW, tiles_y = (g.ny + TT_Y - 1) / TT_Y;
     const int cols = tiles_x * tiles_y;
     const int slots = std::max(1, gather_blocks_v<T, TXW, TYT, GJ>()) * num_sms;  // resident blocks
-    int nzt = (g.nz + BZ - 1) / BZ;                                          // z tiles per column
-    const int waves = (cols * nzt + slots - 1) / slots;
-    nzt = std::min((g.nz + 7) / 8, std::max(nzt, waves * slots / cols));  // at least 8 planes a tile
-    const int bz = (g.nz + nzt - 1) / nzt;
+    const int bz = wave_depth(cols, g.nz, slots);
     const int ntiles = cols * ((g.nz + bz - 1) / bz);
     const int grid = std::min(ntiles, slots);
     k_gather_tma<T, TXW, TYT, GJ><<<grid, dim3(TXW / 2, TYT), smem, s>>>(tm_wx, tm_wy, tm_wz, tm_gj, g, gout, tiles_x,

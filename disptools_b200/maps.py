@@ -26,11 +26,10 @@ import torch
 
 from . import _native as N
 from . import io as fio
-from . import torch_ops
 
 # Clamp modes of dtb_log_jacobian_accumulate_device
 CLAMP_THRESHOLD = 0   # values outside [epsilon, 1e9] become epsilon
-CLAMP_REGULARISE = 1  # values below epsilon become epsilon
+CLAMP_REGULARISE = 1  # values below epsilon become epsilon (fields: dtb_log_jacobian_field_device)
 
 
 def _stream(t: torch.Tensor) -> int:
@@ -128,11 +127,26 @@ def average_jacobian_from_displacements(fields, epsilon: float = 1e-5,
     ``spacing``), each regularised at epsilon.  The Jacobians are computed
     in FP64 with the reference stencil."""
     items = _expand(fields)
-    Js = []
-    for item in items:
+    if not items:
+        raise ValueError("no maps")
+    acc = None
+    for i, item in enumerate(items):
         f, sp = _load_field(item, spacing)
-        fd = _device_tensor(f).to(torch.float64).contiguous()
-        Js.append(torch_ops.jacobian_raw(fd, sp))
+        fd = _device_tensor(f)
+        if fd.dtype not in (torch.float32, torch.float64):
+            fd = fd.to(torch.float64)
+        if fd.dim() != 4 or fd.shape[0] != 3:
+            raise ValueError("field must have shape (3, nz, ny, nx)")
+        if acc is None:
+            acc = torch.empty(fd.shape[1:], dtype=torch.float64, device=fd.device)
+        elif fd.shape[1:] != acc.shape:
+            raise ValueError("all maps must have the same shape")
+        _, nz, ny, nx = fd.shape
+        # One pass a field: its Jacobian in FP64, the log added to the sum;
+        # the last leaves the mean.
+        with torch.cuda.device(fd.device):
+            N.check(N.lib.dtb_log_jacobian_field_device(
+                _prec(fd), nx, ny, nz, *map(float, sp), fd.data_ptr(), float(epsilon), i == 0,
+                i == len(items) - 1, 1.0 / len(items), acc.data_ptr(), _stream(fd)))
     host = not any(isinstance(f, torch.Tensor) for f in items)
-    out = _geometric_mean(Js, CLAMP_REGULARISE, epsilon)
-    return out.cpu().numpy() if host else out
+    return acc.cpu().numpy() if host else acc

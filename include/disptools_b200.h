@@ -295,15 +295,9 @@ int dtb_jacobian_adjoint_cof_device(
  * cudaMalloc / cudaFree can synchronise the device and stall a loop with a
  * deadline), processes whose device memory another allocator has already
  * reserved, and runtimes that hand the library pointers into memory they
- * manage.  Its launch descriptor and tile table live in a 65 KiB array in
- * device memory that belongs to the library and is held by every GPU that
- * loads it until the process exits.  The first call on a device looks up
- * that array's address (cudaGetSymbolAddress), so make it before any stream
- * capture.  Volumes up to 16384 tiles of 32 x 8 x 32 voxels (512^3) are
- * accepted; larger ones return DTB_ERR_ARGUMENT before any device work.
- * All calls on a device share the array and it keeps the last call's
- * contents: calls whose work overlaps on the GPU race, so consecutive calls
- * on one device must use one stream or be ordered by an event. */
+ * manage.  The kernel takes its geometry as a parameter.  Volumes up to
+ * 16384 tiles of 32 x 8 x 32 voxels (512^3) are accepted; larger ones return
+ * DTB_ERR_ARGUMENT before any device work.  Enqueued on `stream`, no wait. */
 int dtb_jacobian_device_noalloc(
     int precision, int order, size_t nx, size_t ny, size_t nz, double dx, double dy, double dz,
     const void *field, void *J, void *stream);
@@ -380,6 +374,14 @@ int dtb_log_jacobian_accumulate_device(int precision, int mode, size_t n, double
 /* out[i] = exp(scale * acc[i]): the geometric mean, scale = 1 / maps. */
 int dtb_exp_mean_device(int precision, size_t n, double scale, const double *acc, void *out,
                         void *stream);
+/* average_jacobian_from_displacements a field at a time: computes the field's
+ * Jacobian map in FP64 (fourth order, `field` [3][nz][ny][nx] of the
+ * precision's element type), replaces values below epsilon by epsilon, and
+ * adds its log to acc [nz][ny][nx].  The first field (`first`) starts the sum
+ * without reading acc; the last (`last`) leaves exp(scale * sum) in acc. */
+int dtb_log_jacobian_field_device(int precision, size_t nx, size_t ny, size_t nz, double dx, double dy, double dz,
+                                  const void *field, double epsilon, int first, int last, double scale,
+                                  double *acc, void *stream);
 
 /* ------------------------------------------------------------------ */
 /* Field files (host)                                                  */

@@ -115,3 +115,41 @@ def test_extension_jacobian_matches(golden):
     out = np.zeros((10, 10, 10))
     _disptools.jacobian((1.0, 1.0, 1.0), g["sin10_field"], out)
     np.testing.assert_array_equal(out, g["sin10_J"])
+
+
+@pytest.mark.parametrize("order", [4, 2])
+@pytest.mark.parametrize("shape", [(3, 3, 3), (4, 7, 33), (33, 8, 31), (5, 9, 65), (70, 17, 45), (2 * 32 + 3, 25, 99)])
+def test_any_layout_kernel_at_tile_edges(oracle, oracle_pd2, shape, order):
+    """The element-wise kernel (odd widths; a base off a 16-byte boundary;
+    second order) around its 32 x 8 tiles: FP64 to 1e-12 of the oracle, FP32
+    to 2e-5, and the same bits whatever the base."""
+    torch = _torch()
+    from disptools_b200 import torch_ops
+    rng = np.random.default_rng(sum(shape))
+    f = rng.normal(scale=0.2, size=(3,) + shape)
+    sp = (0.9, 1.2, 1.05)
+    ref = (oracle if order == 4 else oracle_pd2).jacobian(f, sp)
+    for dtype, tol in ((torch.float64, 1e-12), (torch.float32, 2e-5)):
+        fd = torch.from_numpy(f).to(dtype).cuda()
+        J = torch_ops.jacobian_raw(fd, sp, order)
+        assert rel_err(J.double().cpu().numpy(), ref) <= tol
+        off = torch.empty(fd.numel() + 1, dtype=dtype, device="cuda")[1:].view(fd.shape)
+        off.copy_(fd)
+        J2 = torch_ops.jacobian_raw(off, sp, order)
+        if shape[2] % 2:
+            assert torch.equal(J, J2)
+        else:
+            assert rel_err(J2.double().cpu().numpy(), ref) <= tol
+
+
+def test_any_layout_kernel_keeps_infinities_local(oracle):
+    """An infinite value reaches only the voxels whose schemes read it, also
+    on the second-order outer layers."""
+    torch = _torch()
+    from disptools_b200 import torch_ops
+    f = np.random.default_rng(4).normal(scale=0.1, size=(3, 9, 11, 13))
+    f[1, 4, 5, 3] = np.inf
+    with np.errstate(invalid="ignore"):
+        ref = oracle.jacobian(f)
+    J = torch_ops.jacobian_raw(torch.from_numpy(f).cuda()).cpu().numpy()
+    np.testing.assert_array_equal(np.isfinite(J), np.isfinite(ref))

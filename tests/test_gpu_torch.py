@@ -244,3 +244,25 @@ def test_cof_entry_points_reject_unsupported_layouts():
                                                gJ.data_ptr(), g.data_ptr(), s)
     assert rc == -1 and N.lib.disptools_has_error()
     N.lib.disptools_clear_error()
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 3), (6, 18, 33), (34, 17, 35), (5, 16, 67)])
+@pytest.mark.parametrize("order", [4, 2])
+def test_adjoint_of_odd_widths(oracle, oracle_pd2, shape, order):
+    """Padded weights and unpaired stores: <w, dJ[v]> = <adj w, v> with the
+    directional derivative of the oracle's (cubic) map by central differences,
+    whose only error is h^2 det(grad v) ~ 1e-8 and rounding / h ~ 1e-12."""
+    import torch
+    from disptools_b200 import torch_ops
+    rng = np.random.default_rng(sum(shape) + order)
+    u, v = rng.normal(scale=0.2, size=(2, 3) + shape)
+    w = rng.standard_normal(shape)
+    sp = (0.9, 1.1, 1.3)
+    o = oracle if order == 4 else oracle_pd2
+    h = 1e-4
+    dJ = (o.jacobian(u + h * v, sp) - o.jacobian(u - h * v, sp)) / (2 * h)
+    scale = np.sum(np.abs(w * dJ))
+    for dtype, tol in ((torch.float64, 1e-7), (torch.float32, 1e-5)):
+        g = torch_ops.jacobian_adjoint_raw(torch.from_numpy(u).to(dtype).cuda(), torch.from_numpy(w).to(dtype).cuda(),
+                                           sp, order).double().cpu().numpy()
+        assert abs(np.sum(g * v) - np.sum(w * dJ)) <= tol * scale
