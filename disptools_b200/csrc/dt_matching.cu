@@ -28,17 +28,21 @@
 // positions), and its last block folds the block sums.  The gradient kernel
 // forms each cell's 24 contributions to its corners in shared memory; every
 // grid point then adds the shares of its 8 cells in a fixed order, so the
-// gradient needs no atomics and is deterministic.  The step control runs on
-// the host in the reference's order; each cost evaluation returns its FP64
-// sum and the maximum voxel error.  The conversions between displacements
-// and positions run on the device too.
+// gradient needs no atomics and is deterministic.  The step control
+// (:408-557) runs on the device, in the thread that folds a cost's block
+// sums, and the kernels read from it which positions they work on and
+// whether there is anything to do, so the host queues steps ahead and reads
+// the state a batch later: a host that is late no longer stalls the device.
+// The conversions between displacements and positions run on the device too.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "dt_internal.h"
@@ -58,12 +62,106 @@ struct MatchArgs {
     float eps, zeta;
 };
 
-// A trial move p - alpha dp, formed where the cost kernel stages a plane.
+// A trial move p - alpha dp, formed where the cost kernel stages a plane (the
+// kernel takes alpha and next from the state).
 struct MoveArgs {
     const float *step;
     float alpha;
     float *next;  // moved positions of the points a block owns
 };
+
+// The optimiser's state (:408-557), in device memory.  A step is a gradient
+// launch, which works when `need_gradient`, and a cost launch at `alpha`,
+// whose last block decides what comes next.
+enum MatchPhase {
+    MP_START = 0,   // cost of the initial positions
+    MP_TRIAL = 1,   // first trial of an iteration
+    MP_DOUBLE = 2,  // first iteration: doubling while the cost falls
+    MP_MOVE = 3,    // first iteration: the last doubling but one again (its cost is known)
+    MP_HALVE = 4,   // halving while the cost rises
+};
+struct alignas(16) MatchState {
+    // What every block reads, as one 16-byte load.
+    float alpha;
+    int cur;  // which of the two position buffers holds the current ones
+    int done, need_gradient;
+    float Hcur, Hmark;
+    int phase, pad;
+    double max_error;  // of the last cost evaluated, accepted or not (:103, :176-179)
+    long long it, gradients, costs;
+};
+__device__ __forceinline__ int4 match_head(const MatchState *st) { return __ldcg(reinterpret_cast<const int4 *>(st)); }
+struct MatchLimits {
+    long long it_max;
+    double epsilon;
+};
+
+// The next iteration, or the end.
+__device__ inline void match_next(MatchState *st, const MatchLimits &lim) {
+    if (st->it < lim.it_max && st->alpha > 0.000000001 && st->max_error > lim.epsilon) {
+        st->Hmark = st->Hcur;
+        st->need_gradient = 1;
+        st->phase = MP_TRIAL;
+    } else {
+        st->done = 1;
+    }
+}
+__device__ inline void match_accept(MatchState *st, float Hnext, const MatchLimits &lim) {
+    if (st->alpha > 0.000000001) {
+        st->cur ^= 1;
+        st->Hcur = Hnext;
+        st->it++;
+    }
+    match_next(st, lim);
+}
+// Step control after a cost evaluation (sum H, maximum voxel error M), one
+// thread, in the reference's order.
+__device__ inline void match_control(MatchState *st, double H, double M, const MatchLimits &lim) {
+    const float nH = (float) H;
+    st->gradients += st->need_gradient;
+    st->need_gradient = 0;
+    if (st->phase == MP_MOVE) {  // only the moved positions were wanted
+        match_accept(st, st->Hmark, lim);
+        return;
+    }
+    st->costs++;
+    st->max_error = M;
+    switch (st->phase) {
+    case MP_START:
+        st->Hcur = nH;
+        match_next(st, lim);
+        return;
+    case MP_TRIAL:
+        if (nH < st->Hmark) {
+            if (st->it == 0) {
+                st->Hmark = nH;
+                st->alpha *= 2.0f;
+                st->phase = MP_DOUBLE;
+            } else {
+                st->alpha = (float) ((double) st->alpha * 1.05);  // float times a double constant, as in :476
+                match_accept(st, nH, lim);
+            }
+            return;
+        }
+        break;
+    case MP_DOUBLE:
+        if (nH < st->Hmark) {
+            st->Hmark = nH;
+            st->alpha *= 2.0f;
+        } else {
+            st->alpha *= 0.5f;
+            st->phase = MP_MOVE;
+        }
+        return;
+    default: break;
+    }
+    if (nH > st->Hmark && st->alpha > .000000001) {
+        st->alpha *= 0.5f;
+        st->phase = MP_HALVE;
+    } else {
+        match_accept(st, nH, lim);
+    }
+}
 
 // Tiles of the z-marching kernels.  A block of 256 threads covers 32
 // columns along x and a few rows along y over a run of planes.  Every plane
@@ -212,11 +310,17 @@ __device__ __forceinline__ void plane_commit(const MatchArgs &a, const MoveArgs 
 // ahead.  Per block: the FP64 sum of the cell costs and the maximum voxel
 // error |sum J - 8 V| / 8 (in float, :176-179), each in a fixed order; the
 // last block to finish folds the block results in a fixed order into
-// *result and resets the counter.
+// the step control's input and resets the counter.  `pos0` and `pos1` are the
+// two position buffers.
 template <bool MOVE>
-__global__ void __launch_bounds__(MT_THREADS) k_match_cost(MatchArgs a, MoveArgs m, int zc, double2 *partial,
-                                                           unsigned *counter, double2 *result) {
+__global__ void __launch_bounds__(MT_THREADS) k_match_cost(MatchArgs a, float *pos0, float *pos1, const float *step,
+                                                           int zc, double2 *partial, unsigned *counter,
+                                                           MatchState *st, MatchLimits lim) {
     using B = CostBox;
+    const int4 head = match_head(st);
+    if (head.z) return;  // done
+    a.pos = head.y ? pos1 : pos0;
+    const MoveArgs m{step, __int_as_float(head.x), head.y ? pos0 : pos1};
     __shared__ float pl[3][B::ELEMS];
     __shared__ double rs[MT_THREADS / 32], rm[MT_THREADS / 32];
     __shared__ bool last;
@@ -306,6 +410,8 @@ __global__ void __launch_bounds__(MT_THREADS) k_match_cost(MatchArgs a, MoveArgs
     __syncthreads();
     if (!last) return;
     __threadfence();
+    MatchState now;  // on its way during the fold
+    if (tid == 0) now = *st;
     s = 0.0;
     mx = 0.0;
     for (unsigned b = tid; b < nblocks; b += MT_THREADS) {
@@ -329,8 +435,9 @@ __global__ void __launch_bounds__(MT_THREADS) k_match_cost(MatchArgs a, MoveArgs
             bs += rs[i];
             bm = fmax(bm, rm[i]);
         }
-        *result = make_double2(bs, bm);
         *counter = 0u;
+        match_control(&now, bs, bm, lim);
+        *st = now;
     }
 }
 
@@ -373,8 +480,12 @@ __device__ __forceinline__ void edge_terms(float cE, const float (&w)[8], const 
 // the shares the layer below left at the upper corners (plane k complete, in
 // a fixed order) and keeps the upper corners' shares for plane k + 1.  No
 // atomics, no zeroing pass.
-__global__ void __launch_bounds__(MT_THREADS) k_match_grad(MatchArgs a, int zc, float *step) {
+__global__ void __launch_bounds__(MT_THREADS) k_match_grad(MatchArgs a, const float *pos0, const float *pos1, int zc,
+                                                           float *step, const MatchState *st) {
     using B = GradBox;
+    const int4 head = match_head(st);
+    if (head.z || !head.w) return;  // done, or no gradient wanted
+    a.pos = head.y ? pos1 : pos0;
     __shared__ float pl[3][B::ELEMS];
     __shared__ float cs[24][MG_CELLS];  // [corner * 3 + field][cell]
     const int tid = threadIdx.x;
@@ -493,13 +604,6 @@ __global__ void __launch_bounds__(MT_THREADS) k_match_grad(MatchArgs a, int zc, 
     }
 }
 
-// The move p - alpha dp (:525-530) of every grid point.
-__global__ void k_match_move(const float *cur, const float *step, float alpha, float *next, long long n3) {
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n3;
-         i += (long long) gridDim.x * blockDim.x)
-        next[i] = cur[i] - alpha * step[i];
-}
-
 // Positions in voxel units from the initial field, and the cell targets
 // from the lowest voxel of each cell (:740-756, the same roundings).
 __global__ void k_match_prepare(const double *field, const double *J, int nx, int ny, int nz, double dx, double dy,
@@ -554,31 +658,78 @@ void report(int line, const char *function, const char *message) {
         }                                                           \
     } while (0)
 
-struct DeviceBuffers {
-    std::vector<void *> p;
-    ~DeviceBuffers() {
-        for (void *q : p) cudaFree(q);
+// The solve's device memory: one allocation, carved up.
+struct Slab {
+    char *base = nullptr;
+    size_t bytes = 0;
+    ~Slab() {
+        if (base) cudaFree(base);
+    }
+    // Offset of n more elements.
+    template <typename U>
+    size_t add(size_t n) {
+        const size_t at = (bytes + 255) & ~size_t(255);
+        bytes = at + n * sizeof(U);
+        return at;
+    }
+    bool allocate() {
+        if (cudaMalloc(&base, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            base = nullptr;
+        }
+        return base != nullptr;
     }
     template <typename U>
-    U *take(size_t n) {
-        void *q = nullptr;
-        if (cudaMalloc(&q, n * sizeof(U)) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        p.push_back(q);
-        return static_cast<U *>(q);
+    U *at(size_t off) const {
+        return reinterpret_cast<U *>(base + off);
     }
 };
 
-// Four timing events, destroyed with the object.
+// Pinned copies of the state, two a solve (one per batch of steps in flight).
+// Kept for later solves: as many as have run at the same time.
+struct HostStates {
+    MatchState *p = nullptr;
+    HostStates() {
+        {
+            std::lock_guard<std::mutex> lock(mutex());
+            if (!spare().empty()) {
+                p = spare().back();
+                spare().pop_back();
+                return;
+            }
+        }
+        if (cudaHostAlloc(&p, 2 * sizeof(MatchState), cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    ~HostStates() {
+        if (!p) return;
+        std::lock_guard<std::mutex> lock(mutex());
+        spare().push_back(p);
+    }
+    HostStates(const HostStates &) = delete;
+    HostStates &operator=(const HostStates &) = delete;
+
+private:
+    static std::mutex &mutex() {
+        static std::mutex m;
+        return m;
+    }
+    static std::vector<MatchState *> &spare() {
+        static std::vector<MatchState *> v;
+        return v;
+    }
+};
+
+// Events, destroyed with the object: three for timing, two that follow a batch.
 struct Events {
-    cudaEvent_t e[4] = {};
-    bool create() {
-        for (cudaEvent_t &x : e)
-            if (cudaEventCreate(&x) != cudaSuccess) {
+    cudaEvent_t e[5] = {};
+    bool create(bool timing) {
+        for (int i = timing ? 0 : 3; i < 5; ++i)
+            if (cudaEventCreateWithFlags(&e[i], i < 3 ? cudaEventDefault : cudaEventDisableTiming) != cudaSuccess) {
                 cudaGetLastError();
-                x = nullptr;
+                e[i] = nullptr;
                 return false;
             }
         return true;
@@ -620,141 +771,131 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
     const dtb_params &p = *params;
     const long long n = (long long) (nx * ny * nz);
     const long long cells = (long long) (nx - 1) * (ny - 1) * (nz - 1);
-    DeviceBuffers b;
-    // Positions (current and moved) and the gradient step, [3][n] each.
-    float *cur = b.take<float>(3 * n), *next = b.take<float>(3 * n), *step = b.take<float>(3 * n);
-    float *tv = b.take<float>(cells);
-    double *dfield = device ? field : b.take<double>(3 * n);
-    const double *dJ = device ? J : b.take<double>(n);
     // Launch shapes: 32 x 8 cell columns (cost) or 32 x 6 point columns
-    // (gradient) per block, runs of zc planes, about eight blocks per SM in all.
+    // (gradient) per block, runs of zc planes.
     const int ncx = (int) nx - 1, ncy = (int) ny - 1, ncz = (int) nz - 1;
-    auto zrun = [](long long tiles, int depth) {
-        const long long want = 148 * 8;
-        return (int) std::max<long long>(4, std::min<long long>(depth, (tiles * depth + want - 1) / want));
-    };
-    const int zc_cost = zrun((long long) ((ncx + MT_X - 1) / MT_X) * ((ncy + MC_Y - 1) / MC_Y), ncz);
-    const int zc_grad = zrun((long long) (((int) nx + MT_X - 1) / MT_X) * (((int) ny + MG_Y - 1) / MG_Y), (int) nz);
+    const long long cost_tiles = (long long) ((ncx + MT_X - 1) / MT_X) * ((ncy + MC_Y - 1) / MC_Y);
+    const long long grad_tiles = (long long) (((int) nx + MT_X - 1) / MT_X) * (((int) ny + MG_Y - 1) / MG_Y);
+    // Cost: about eight blocks per SM in all, whose start-up then overlaps (at
+    // 128^3 43.7 us; one wave of 22-layer runs 48.7 us), runs of at least four
+    // layers unless that leaves SMs without a block.
+    const int zc_cost = (int) std::max(std::min(4ll, std::max(1ll, cost_tiles * ncz / 148)),
+                                       std::min<long long>(ncz, (cost_tiles * ncz + 148 * 8 - 1) / (148 * 8)));
+    // Gradient: two blocks fit on an SM and each run also forms the layer below
+    // it, so the depth whose busiest SM has least to do; a block alone on its
+    // SM runs about 1.5 times as fast as one of two.  At 96^3 runs of 16 layers
+    // (two blocks an SM) take 42.9 us, runs of 4 (eight) 49.6 us.
+    int zc_grad = 1;
+    double best = 1e300;
+    for (int zc = std::min((int) nz, 64); zc >= 1; --zc) {
+        const long long q = (grad_tiles * (((int) nz + zc - 1) / zc) + 147) / 148;
+        const double t = (zc + 2) * ((double) (q / 2 * 2) + (q % 2 ? 1.3 : 0.0));
+        if (t < best) {
+            best = t;
+            zc_grad = zc;
+        }
+    }
     const dim3 cost_grid((ncx + MT_X - 1) / MT_X, (ncy + MC_Y - 1) / MC_Y, (ncz + zc_cost - 1) / zc_cost);
     const dim3 grad_grid(((int) nx + MT_X - 1) / MT_X, ((int) ny + MG_Y - 1) / MG_Y, ((int) nz + zc_grad - 1) / zc_grad);
-    const int cost_blocks = (int) (cost_grid.x * cost_grid.y * cost_grid.z);
-    double2 *partial = b.take<double2>(cost_blocks + 1);
-    unsigned *counter = b.take<unsigned>(1);
-    if (!cur || !next || !step || !tv || !dfield || !dJ || !partial || !counter) {
+    const size_t cost_blocks = (size_t) cost_grid.x * cost_grid.y * cost_grid.z;
+    // Positions (two buffers) and the gradient step, [3][n] each.
+    Slab b;
+    const size_t o_pos0 = b.add<float>(3 * n), o_pos1 = b.add<float>(3 * n), o_step = b.add<float>(3 * n);
+    const size_t o_tv = b.add<float>(cells), o_partial = b.add<double2>(cost_blocks), o_state = b.add<MatchState>(1);
+    const size_t o_counter = b.add<unsigned>(1);
+    const size_t o_field = device ? 0 : b.add<double>(3 * n), o_J = device ? 0 : b.add<double>(n);
+    HostStates host;
+    Events ev;
+    const bool prof = profiling_on();
+    if (!b.allocate() || !host.p || !ev.create(prof)) {
         report(__LINE__, __func__, "cannot allocate device buffers");
         return DTB_ERR_ALLOC;
     }
+    float *const pos[2] = {b.at<float>(o_pos0), b.at<float>(o_pos1)}, *const step = b.at<float>(o_step);
+    float *const tv = b.at<float>(o_tv);
+    double2 *const partial = b.at<double2>(o_partial);
+    MatchState *const st = b.at<MatchState>(o_state);
+    unsigned *const counter = b.at<unsigned>(o_counter);  // finished blocks of the cost launch
+    double *const dfield = device ? field : b.at<double>(o_field);
+    const double *const dJ = device ? J : b.at<double>(o_J);
+    MatchState init;
+    std::memset(&init, 0, sizeof init);
+    init.alpha = 1.0f;
+    init.max_error = DBL_MAX;
+    const MatchLimits lim{p.it_max, p.epsilon};
+    host.p[0] = init;
     M_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
+    M_CUDA(cudaMemcpyAsync(st, &host.p[0], sizeof init, cudaMemcpyHostToDevice, s));
     if (!device) {
         M_CUDA(cudaMemcpyAsync(dfield, field, 3 * n * sizeof(double), cudaMemcpyHostToDevice, s));
         M_CUDA(cudaMemcpyAsync(const_cast<double *>(dJ), J, n * sizeof(double), cudaMemcpyHostToDevice, s));
     }
-    k_match_prepare<<<grid_for(n), 256, 0, s>>>(dfield, dJ, (int) nx, (int) ny, (int) nz, dx, dy, dz, cur, cur + n,
-                                                cur + 2 * n, tv);
+    k_match_prepare<<<grid_for(n), 256, 0, s>>>(dfield, dJ, (int) nx, (int) ny, (int) nz, dx, dy, dz, pos[0],
+                                                pos[0] + n, pos[0] + 2 * n, tv);
     count_launch();
     M_CUDA(cudaGetLastError());
 
-    const float eps = (float) p.delta, zeta = (float) p.zeta;
-    double2 h_res;
-    double max_voxel_error = DBL_MAX;
-    // Profiling (dtb_set_profiling): events around the gradient and cost
-    // launches, read after the host wait that follows every cost.
-    Events ev;
-    const bool prof = profiling_on() && ev.create();
-    bool grad_timed = false;
-    // Cost of the current positions (alpha < 0) or of the positions moved by
-    // alpha, which are then in `next`; updates max_voxel_error like the
-    // reference's global (:103, :176-179).
-    auto cost = [&](float alpha, float *H) -> int {
-        const MatchArgs a{cur, tv, (int) nx, (int) ny, (int) nz, (unsigned) n, eps, zeta};
-        double2 *res = partial + cost_blocks;
-        if (prof) M_CUDA(cudaEventRecord(ev.e[2], s));
-        if (alpha < 0.0f) {
-            k_match_cost<false><<<cost_grid, MT_THREADS, 0, s>>>(a, MoveArgs{}, zc_cost, partial, counter, res);
-        } else {
-            const MoveArgs mv{step, alpha, next};
-            k_match_cost<true><<<cost_grid, MT_THREADS, 0, s>>>(a, mv, zc_cost, partial, counter, res);
-        }
-        count_launch();
-        M_CUDA(cudaGetLastError());
-        if (prof) M_CUDA(cudaEventRecord(ev.e[3], s));
-        M_CUDA(cudaMemcpyAsync(&h_res, res, sizeof h_res, cudaMemcpyDeviceToHost, s));
-        M_CUDA(cudaStreamSynchronize(s));
-        *H = (float) h_res.x;
-        max_voxel_error = h_res.y;
-        if (prof) {
-            float ms = 0.0f;
-            if (grad_timed && cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]) == cudaSuccess)
-                profile_match(PROF_MATCH_GRAD, ms);
-            if (cudaEventElapsedTime(&ms, ev.e[2], ev.e[3]) == cudaSuccess) profile_match(PROF_MATCH_COST, ms);
-            grad_timed = false;
-        }
-        return DTB_OK;
-    };
-    auto grads = [&]() -> int {
-        const MatchArgs a{cur, tv, (int) nx, (int) ny, (int) nz, (unsigned) n, eps, zeta};
-        if (prof) M_CUDA(cudaEventRecord(ev.e[0], s));
-        k_match_grad<<<grad_grid, MT_THREADS, 0, s>>>(a, zc_grad, step);
-        count_launch();
-        M_CUDA(cudaGetLastError());
-        if (prof) {
-            M_CUDA(cudaEventRecord(ev.e[1], s));
-            grad_timed = true;
-        }
-        return DTB_OK;
-    };
-    auto move = [&](float alpha) -> int {
-        k_match_move<<<grid_for(3 * n), 256, 0, s>>>(cur, step, alpha, next, 3 * n);
-        count_launch();
-        M_CUDA(cudaGetLastError());
-        return DTB_OK;
-    };
-#define M_DO(x)                      \
-    do {                             \
-        const int rc_ = (x);         \
-        if (rc_ != DTB_OK) return rc_; \
-    } while (0)
+    const MatchArgs a{nullptr, tv, (int) nx, (int) ny, (int) nz, (unsigned) n, (float) p.delta, (float) p.zeta};
+    k_match_cost<false><<<cost_grid, MT_THREADS, 0, s>>>(a, pos[0], pos[1], step, zc_cost, partial, counter, st, lim);
+    count_launch();
+    M_CUDA(cudaGetLastError());
 
-    // The optimiser of :408-557.
-    const long long maxit = p.it_max;
-    float alpha = 1.0f, Hcur = 0.0f, Hmark, nH;
-    M_DO(cost(-1.0f, &Hcur));
-    long long itnum = 0;
-    while (itnum < maxit && alpha > 0.000000001 && max_voxel_error > p.epsilon) {
-        Hmark = Hcur;
-        M_DO(grads());
-        M_DO(cost(alpha, &nH));  // move and cost in one pass
-        float Hnext;
-        if (nH < Hmark) {
-            if (itnum == 0) {
-                while (nH < Hmark) {
-                    Hmark = nH;
-                    alpha *= 2.0f;
-                    M_DO(cost(alpha, &nH));
-                }
-                alpha *= 0.5f;
-                M_DO(move(alpha));
-                Hnext = Hmark;
-            } else {
-                Hnext = nH;
-                alpha = (float) ((double) alpha * 1.05);  // float times a double constant, as in :476
-            }
-        } else {
-            while (nH > Hmark && alpha > .000000001) {
-                alpha *= 0.5f;
-                M_DO(cost(alpha, &nH));
-            }
-            Hnext = nH;
+    // Batches of steps; batch r leaves the state in host copy r % 2 and is
+    // waited for after batch r + 1 has been queued.  Launches after the end
+    // return at once.  Profiling (dtb_set_profiling) runs single steps, waits
+    // for each and counts the launches that did work.
+    const int batch = prof ? 1 : 8;
+    auto enqueue = [&](long long r) -> int {
+        for (int k = 0; k < batch; ++k) {
+            if (prof) M_CUDA(cudaEventRecord(ev.e[0], s));
+            k_match_grad<<<grad_grid, MT_THREADS, 0, s>>>(a, pos[0], pos[1], zc_grad, step, st);
+            count_launch();
+            M_CUDA(cudaGetLastError());
+            if (prof) M_CUDA(cudaEventRecord(ev.e[1], s));
+            k_match_cost<true><<<cost_grid, MT_THREADS, 0, s>>>(a, pos[0], pos[1], step, zc_cost, partial, counter, st, lim);
+            count_launch();
+            M_CUDA(cudaGetLastError());
+            if (prof) M_CUDA(cudaEventRecord(ev.e[2], s));
         }
-        if (alpha > .000000001) {
-            std::swap(cur, next);
-            Hcur = Hnext;
-            itnum++;
+        M_CUDA(cudaMemcpyAsync(&host.p[r & 1], st, sizeof(MatchState), cudaMemcpyDeviceToHost, s));
+        M_CUDA(cudaEventRecord(ev.e[3 + (r & 1)], s));
+        return DTB_OK;
+    };
+    // An iteration's doublings and halvings span the float range at most.
+    const long long max_steps = 400 * (std::max<long long>(p.it_max, 0) + 2);
+    MatchState last = init;
+    auto run = [&]() -> int {
+        int rc = enqueue(0);
+        if (rc != DTB_OK) return rc;
+        for (long long r = 0;; ++r) {
+            if (!prof && (rc = enqueue(r + 1)) != DTB_OK) return rc;
+            M_CUDA(cudaEventSynchronize(ev.e[3 + (r & 1)]));
+            const MatchState now = host.p[r & 1];
+            if (prof) {
+                float ms = 0.0f;
+                if (now.gradients > last.gradients && cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]) == cudaSuccess)
+                    profile_match(PROF_MATCH_GRAD, ms);
+                if (now.costs > last.costs && cudaEventElapsedTime(&ms, ev.e[1], ev.e[2]) == cudaSuccess)
+                    profile_match(PROF_MATCH_COST, ms);
+            }
+            last = now;
+            if (now.done) return DTB_OK;
+            if ((r + 1) * batch > max_steps) {
+                report(__LINE__, __func__, "the solver did not terminate within its step bound");
+                return DTB_ERR_ARGUMENT;
+            }
+            if (prof && (rc = enqueue(r + 1)) != DTB_OK) return rc;
         }
+    };
+    const int rc = run();
+    if (rc != DTB_OK) {
+        cudaStreamSynchronize(s);  // before the memory goes
+        cudaGetLastError();
+        return rc;
     }
-#undef M_DO
 
     // Back to displacements in the caller's layout (:777-787).
+    float *const cur = pos[last.cur];
     k_match_finish<<<grid_for(n), 256, 0, s>>>(cur, cur + n, cur + 2 * n, (int) nx, (int) ny, (int) nz, dx, dy, dz,
                                                dfield);
     count_launch();
@@ -763,13 +904,13 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
     M_CUDA(cudaStreamSynchronize(s));
     if (stats) {
         std::memset(stats, 0, sizeof *stats);
-        stats->iterations = itnum;
-        stats->error = Hcur;
-        stats->max_error = max_voxel_error;
-        stats->eta = alpha;
+        stats->iterations = last.it;
+        stats->error = last.Hcur;
+        stats->max_error = last.max_error;
+        stats->eta = last.alpha;
         stats->precision = DTB_PRECISION_MIXED;
-        stats->reason = itnum >= maxit ? DTB_STOP_IT_MAX
-                                       : (alpha > 0.000000001 ? DTB_STOP_EPSILON : DTB_STOP_ETA);
+        stats->reason = last.it >= p.it_max ? DTB_STOP_IT_MAX
+                                            : (last.alpha > 0.000000001 ? DTB_STOP_EPSILON : DTB_STOP_ETA);
     }
     return DTB_OK;
 }

@@ -106,3 +106,79 @@ def test_matching_profile_counts_kernels():
     g, c = prof["match_gradient"], prof["match_cost"]
     assert g[0] >= 5 and c[0] >= g[0] + 1
     assert g[1] > 0.0 and c[1] > 0.0
+
+
+def _optimiser64(J, params):
+    """The optimiser of src/VolumeMatching3D.c:408-557 on a zero field, unit
+    spacing, cost and gradient in float64 by torch's autograd."""
+    import torch
+    nz, ny, nx = J.shape
+    grid = torch.meshgrid(*[torch.arange(1, n + 1, dtype=torch.float64) for n in (nz, ny, nx)], indexing="ij")
+    pos = torch.stack([grid[1], grid[2], grid[0]])  # y, x, z
+    V = torch.as_tensor(J)[:-1, :-1, :-1]
+    eps, zeta = params["delta"], params["zeta"]
+
+    def cost(p):
+        edge = [p[:, :, 1:] - p[:, :, :-1], p[:, :, :, 1:] - p[:, :, :, :-1], p[:, 1:] - p[:, :-1]]  # along y, x, z
+        s, barrier = 0.0, 0.0
+        for k in (0, 1):
+            for x in (0, 1):
+                for y in (0, 1):
+                    m = [edge[0][:, k:nz - 1 + k, :, x:nx - 1 + x], edge[1][:, k:nz - 1 + k, y:ny - 1 + y],
+                         edge[2][:, :, y:ny - 1 + y, x:nx - 1 + x]]
+                    Jc = torch.linalg.det(torch.stack(m, dim=-1).movedim(0, -2))
+                    s = s + Jc
+                    barrier = barrier + torch.where(Jc < eps, zeta * (Jc - eps) ** 2, torch.zeros_like(Jc))
+        volume = torch.where(V > 0, (s - 8 * V) ** 2, torch.zeros_like(s))
+        return 0.5 * (volume + barrier).sum(), float(((s - 8 * V).abs() / 8).max().detach())
+
+    def trial(g, alpha):
+        h, worst = cost(pos - alpha * g)
+        return float(h), worst
+
+    alpha, it, phases = 1.0, 0, set()
+    H, worst = trial(torch.zeros_like(pos), 0.0)
+    while it < params["it_max"] and alpha > 1e-9 and worst > params["epsilon"]:
+        q = pos.clone().requires_grad_()
+        (g,) = torch.autograd.grad(cost(q)[0], q)
+        mark = H
+        h, worst = trial(g, alpha)
+        step = alpha
+        if h < mark and it == 0:
+            phases.add("double")
+            while h < mark:
+                mark, alpha = h, alpha * 2
+                h, worst = trial(g, alpha)
+            step = alpha = alpha * 0.5
+            h = mark
+        elif h < mark:
+            phases.add("grow")
+            alpha = float(np.float32(alpha) * 1.05)
+        else:
+            while h > mark and alpha > 1e-9:
+                phases.add("halve")
+                alpha *= 0.5
+                h, worst = trial(g, alpha)
+            step = alpha
+        if alpha > 1e-9:
+            pos, H, it = pos - step * g, h, it + 1
+    return pos, it, phases
+
+
+# zeta 1e-3 with a floor of 2 and no volume term (J <= 0): the first step
+# of 1 lowers the cost, so it is doubled; the other start halves it.
+@pytest.mark.parametrize("target, delta, zeta, wanted", [(0.0, 2.0, 1e-3, "double"), (1.2, 1e-3, 10.0, "halve")])
+def test_device_step_control_against_float64(target, delta, zeta, wanted):
+    """The doubling, growing and halving branches of the device's step control
+    against a float64 restatement, for a few iterations (the solver computes
+    in float32)."""
+    J = np.full((4, 5, 6), target)
+    J[2, 2, 3] += 0.3 * (target > 0)
+    params = dict(delta=delta, zeta=zeta, it_max=3, epsilon=9.99e-4)
+    pos, it, phases = _optimiser64(J, params)
+    assert wanted in phases
+    out, st = dt.solve(J, np.ones(J.shape, bool), algorithm="matching", **params)
+    assert st["iterations"] == it
+    z, y, x = np.meshgrid(*[np.arange(1, n + 1) for n in J.shape], indexing="ij")
+    ref = np.stack([pos[1].numpy() - x, pos[0].numpy() - y, pos[2].numpy() - z])
+    assert np.max(np.abs(out - ref)) <= 1e-4
