@@ -217,6 +217,10 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
         const int se = slot >= 2 ? slot - 2 : slot - 2 + JA_NS;
         slot = slot + 1 < JA_NS ? slot + 1 : 0;
         if (ze < z0 || !in_xy) continue;
+        // What the epilogue reads, on its way during the stencil.
+        T pre = T(0);
+        if constexpr (EPI == JAC_WEIGHTS) pre = __ldg(out.gJ + off);
+        if constexpr (EPI == JAC_LOG) pre = out.first ? T(0) : out.acc[off];
         const bool plane_in = ze >= 2 && ze <= g.nz - 3;
         T a[3][3];
         stencil_voxel<TI, T>(ring + se * JA_PLANE + own, zq, x, y, ze, g, ih, tile_in && plane_in,
@@ -226,11 +230,10 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
         } else if constexpr (EPI == JAC_LOG) {
             double j = (double) det_i_plus<T>(a);
             j = j < out.eps ? out.eps : j;
-            double s = log(j);
-            if (!out.first) s = out.acc[off] + s;
+            const double s = pre + log(j);
             out.acc[off] = out.last ? exp(out.scale * s) : s;
         } else {
-            const T w = out.gJ[off];
+            const T w = pre;
             T *W = out.W + (ze * out.wzs + y * out.wys + x);
             a[0][0] += T(1);
             a[1][1] += T(1);
