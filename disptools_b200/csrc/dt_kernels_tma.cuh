@@ -341,21 +341,137 @@ __device__ __forceinline__ void greedy_prefetch_stale(T *out, int tid, int nth, 
     cp_async_commit();
 }
 
+// One-sided differences with every FP32 rounding stated (the contraction of
+// fd_fwd and fd_bwd that the compiler chose in the trial kernel).
+template <typename T>
+__device__ __forceinline__ T fd_fwd_rn(T a0, T p1, T p2, T ih) {
+    if constexpr (sizeof(T) == 4) return __fmul_rn(__fmaf_rn(-.5f, p2, __fmaf_rn(2.f, p1, __fmul_rn(-1.5f, a0))), ih);
+    else return fd_fwd<T>(a0, p1, p2, ih);
+}
+template <typename T>
+__device__ __forceinline__ T fd_bwd_rn(T a0, T m1, T m2, T ih) {
+    if constexpr (sizeof(T) == 4) return __fmul_rn(__fmaf_rn(.5f, m2, __fmaf_rn(1.5f, a0, -2.f * m1)), ih);
+    else return fd_bwd<T>(a0, m1, m2, ih);
+}
+
+template <typename T>
+__device__ __forceinline__ typename PairOf<T>::type fd_fwd_pair(typename PairOf<T>::type a0, typename PairOf<T>::type p1,
+                                                                typename PairOf<T>::type p2, T ih) {
+    if constexpr (sizeof(T) == 4)
+        return p_mul(p_fma(p_splat(-.5f), p2, p_fma(p_splat(2.f), p1, p_mul(p_splat(-1.5f), a0))), p_splat(ih));
+    else return typename PairOf<T>::type{fd_fwd<T>(a0.x, p1.x, p2.x, ih), fd_fwd<T>(a0.y, p1.y, p2.y, ih)};
+}
+template <typename T>
+__device__ __forceinline__ typename PairOf<T>::type fd_bwd_pair(typename PairOf<T>::type a0, typename PairOf<T>::type m1,
+                                                                typename PairOf<T>::type m2, T ih) {
+    if constexpr (sizeof(T) == 4)
+        return p_mul(p_fma(p_splat(.5f), m2, p_fma(p_splat(1.5f), a0, p_mul(p_splat(-2.f), m1))), p_splat(ih));
+    else return typename PairOf<T>::type{fd_bwd<T>(a0.x, m1.x, m2.x, ih), fd_bwd<T>(a0.y, m1.y, m2.y, ih)};
+}
+
+// The Jacobian matrices minus I of a pair of voxels of which at least one of
+// the warp's lies in the volume's two outer layers.  There every scheme is
+// second order (schemes_at): central, or one-sided along the axes where the
+// voxel lies on a face; the others take the fourth-order differences.  Both
+// central schemes are one expression of the first and second differences,
+// with per-voxel weights, and the second difference dropped (not multiplied
+// by zero: it may be infinite) where the scheme is second order; each rounds
+// as its own expression does (FP32 d1 k1 + d2 k2 fused, or d1 (ih / 2); FP64
+// ((d1 w1) - d2 / 12) ih half, with w1 = 2/3 and half = 1, or w1 = 1, d2 = 0
+// and half = 1/2).  Only the lanes on a face recompute that axis one-sided.
+// A case analysis per voxel here held up whole blocks: with every voxel of
+// 256^3 sent through the fourth-order path the trial took 45 us less.
+// Arguments as stencil_pair's; the second voxel's matrix is meaningless when
+// x + 1 lies outside the volume.
+template <typename T, int TMA_PX, int TMA_PLANE>
+__device__ __forceinline__ void stencil_shell(const typename PairOf<T>::type (&zq)[3][5], const T *p0, int x, int y,
+                                              int ze, const Geom &g, const T (&ih)[3], bool row_in,
+                                              typename PairOf<T>::type (&a)[3][3]) {
+    using P2 = typename PairOf<T>::type;
+    const bool f0 = row_in && x >= 2 && x <= g.nx - 3, f1 = row_in && x >= 1 && x <= g.nx - 4;
+    auto central = [&](P2 d1, P2 d2, int ax) -> P2 {
+        const P2 e2 = P2{f0 ? d2.x : T(0), f1 ? d2.y : T(0)};
+        if constexpr (sizeof(T) == 4) {
+            const float k1 = FD<T>::two_thirds * ih[ax], k2n = -FD<T>::one_twelfth * ih[ax], h = ih[ax] * T(.5);
+            return p_fma(d1, make_float2(f0 ? k1 : h, f1 ? k1 : h), p_mul(e2, p_splat(k2n)));
+        } else {
+            const T w0 = f0 ? FD<T>::two_thirds : T(1), w1 = f1 ? FD<T>::two_thirds : T(1);
+            return P2{(d1.x * w0 - e2.x * FD<T>::one_twelfth) * ih[ax] * (f0 ? T(1) : T(.5)),
+                      (d1.y * w1 - e2.y * FD<T>::one_twelfth) * ih[ax] * (f1 ? T(1) : T(.5))};
+        }
+    };
+    auto sub = [](P2 u, P2 v) -> P2 {
+        if constexpr (sizeof(T) == 4) return p_sub(u, v);
+        else return P2{u.x - v.x, u.y - v.y};
+    };
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const T *p = p0 + c * TMA_PLANE;
+        const P2 xc = zq[c][2];
+        const P2 xm = ld_pair(p - 2), xp = ld_pair(p + 2);
+        a[c][0] = central(P2{xc.y - xm.y, xp.x - xc.x}, sub(xp, xm), 0);
+        if (x == 0) a[c][0].x = fd_fwd_rn<T>(xc.x, xc.y, xp.x, ih[0]);
+        if (x == g.nx - 1) a[c][0].x = fd_bwd_rn<T>(xc.x, xm.y, xm.x, ih[0]);
+        if (x == g.nx - 2) a[c][0].y = fd_bwd_rn<T>(xc.y, xc.x, xm.y, ih[0]);
+        const P2 ym1 = ld_pair(p - TMA_PX), yp1 = ld_pair(p + TMA_PX);
+        const P2 ym2 = ld_pair(p - 2 * TMA_PX), yp2 = ld_pair(p + 2 * TMA_PX);
+        a[c][1] = central(sub(yp1, ym1), sub(yp2, ym2), 1);
+        if (y == 0) a[c][1] = fd_fwd_pair<T>(xc, yp1, yp2, ih[1]);
+        if (y == g.ny - 1) a[c][1] = fd_bwd_pair<T>(xc, ym1, ym2, ih[1]);
+        a[c][2] = central(sub(zq[c][3], zq[c][1]), sub(zq[c][4], zq[c][0]), 2);
+        if (ze == 0) a[c][2] = fd_fwd_pair<T>(xc, zq[c][3], zq[c][4], ih[2]);
+        if (ze == g.nz - 1) a[c][2] = fd_bwd_pair<T>(xc, zq[c][1], zq[c][0], ih[2]);
+    }
+}
+
+// det(I + a) of both voxels, rounded as the scalar det_i_plus.  The compiler
+// contracts a packed product and the sum after it even where both state their
+// rounding, so each product here is a fused multiply-add of a -0 it cannot
+// know (exact: it only adds to a rounded product what leaves it alone).
+__constant__ float2 c_negative_zero = {-0.f, -0.f};
+template <typename T>
+__device__ __forceinline__ typename PairOf<T>::type det_pair_rn(const typename PairOf<T>::type (&a)[3][3]) {
+    if constexpr (sizeof(T) == 4) {
+        const float2 one = p_splat(1.f), nz = c_negative_zero;
+        auto mul = [&](float2 u, float2 v) { return p_fma(u, v, nz); };
+        const float2 a11 = p_add(a[0][0], one), a22 = p_add(a[1][1], one), a33 = p_add(a[2][2], one);
+        const float2 c1 = p_sub(mul(a22, a33), mul(a[1][2], a[2][1]));
+        const float2 c2 = p_sub(mul(a[1][0], a33), mul(a[1][2], a[2][0]));
+        const float2 c3 = p_sub(mul(a[1][0], a[2][1]), mul(a22, a[2][0]));
+        return p_fma(a[0][2], c3, p_sub(mul(a11, c1), mul(a[0][1], c2)));
+    } else {
+        T a0[3][3], a1[3][3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                a0[c][ax] = a[c][ax].x;
+                a1[c][ax] = a[c][ax].y;
+            }
+        return typename PairOf<T>::type{det_i_plus<T>(a0), det_i_plus<T>(a1)};
+    }
+}
+
+// Half v of the matrices of a pair.
+template <typename T>
+__device__ __forceinline__ void half_of(const typename PairOf<T>::type (&a)[3][3], int v, T (&m)[3][3]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) m[c][ax] = v ? a[c][ax].y : a[c][ax].x;
+}
+
 // The Jacobian matrices minus I of the two voxels (x, x + 1) of row y of
 // plane ze, each handed to finish(v, a) when the voxel lies in the volume.
 // `jp` is the plane's field box in shared memory ([3][TMA_PY][PX], column lx
 // holds x, row ly holds y); zq holds the two columns' values of planes
 // ze-2 .. ze+2 per component as pairs (x, x + 1).  FP32 folds the spacing into the fourth-order
-// weights; the FP64 path keeps the reference's operation order.  Three
-// evaluators:
-// * rows and planes inside [2, n-3] of a tile whose columns all lie inside
-//   [2, nx-3] use the fourth-order stencil only;
-// * interior rows of a tile that reaches an x end select the scheme per
-//   voxel without branching;
-// * rows or planes on the two outer layers take the general path.
-// The trial kernel keeps the same evaluator inline: calling this function
-// there changes its register allocation (it then spills).  In FP32, a
-// `finish2` functor (not null) takes the first evaluator's two matrices at
+// weights; the FP64 path keeps the reference's operation order.  Two
+// evaluators: rows and planes inside [2, n-3] of a tile whose columns all lie
+// inside [2, nx-3] use the fourth-order stencil only; the others take
+// stencil_shell.  The trial kernel keeps the first inline: calling this
+// function there changes its register allocation (it then spills).  In FP32,
+// a `finish2` functor (not null) takes the first evaluator's two matrices at
 // once, as pairs (x, x + 1) of each entry.
 template <typename T, int TMA_PX, int TMA_PLANE, typename F, typename F2 = std::nullptr_t>
 __device__ __forceinline__ void stencil_pair(const typename PairOf<T>::type (&zq)[3][5], const T *jp, int lx,
@@ -404,68 +520,16 @@ __device__ __forceinline__ void stencil_pair(const typename PairOf<T>::type (&zq
         }
         finish(0, a0);
         finish(1, a1);
-    } else if (row_in) {
-        // Interior row: the scheme depends on x only
-        // (src/jacobian.c:113-241): outer column -> one-sided
-        // in x and second-order central in y, z; penultimate
-        // column -> second-order central; else fourth order.
-#pragma unroll
-        for (int v = 0; v < 2; ++v) {
-            const int xv = x + v;
-            if (xv >= g.nx) continue;
-            const bool xo_lo = xv == 0, xo_hi = xv == g.nx - 1;
-            const bool second = xo_lo || xo_hi || xv == 1 || xv == g.nx - 2;
-            T a[3][3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const T *p = jp + c * TMA_PLANE + ly * TMA_PX + lx + v;
-                const T fx = xo_lo ? fd_fwd<T>(p[0], p[1], p[2], ih[0])
-                                   : (xo_hi ? fd_bwd<T>(p[0], p[-1], p[-2], ih[0])
-                                            : fd_c2<T>(p[1], p[-1], ih[0]));
-                const T cx4 = c4(p[1], p[-1], p[2], p[-2], 0);
-                a[c][0] = second ? fx : cx4;
-                const T cy4 = c4(p[TMA_PX], p[-TMA_PX], p[2 * TMA_PX], p[-2 * TMA_PX], 1);
-                const T cy2 = fd_c2<T>(p[TMA_PX], p[-TMA_PX], ih[1]);
-                a[c][1] = second ? cy2 : cy4;
-                T zv[5];
-#pragma unroll
-                for (int k = 0; k < 5; ++k) zv[k] = v ? zq[c][k].y : zq[c][k].x;
-                const T cz4 = c4(zv[3], zv[1], zv[4], zv[0], 2);
-                const T cz2 = fd_c2<T>(zv[3], zv[1], ih[2]);
-                a[c][2] = second ? cz2 : cz4;
-            }
-            finish(v, a);
-        }
     } else {
+        using P2 = typename PairOf<T>::type;
+        P2 a[3][3];
+        stencil_shell<T, TMA_PX, TMA_PLANE>(zq, jp + ly * TMA_PX + lx, x, y, ze, g, ih, row_in, a);
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
-            const int xv = x + v;
-            if (xv >= g.nx) continue;
-            int kk[3];
-            schemes_at(xv, y, ze, g, kk);
-            T a[3][3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const T *p = jp + c * TMA_PLANE + ly * TMA_PX + lx + v;
-                const T vx[5] = {p[-2], p[-1], p[0], p[1], p[2]};
-                const T vy[5] = {p[-2 * TMA_PX], p[-TMA_PX], p[0], p[TMA_PX], p[2 * TMA_PX]};
-#pragma unroll
-                for (int ax = 0; ax < 3; ++ax) {
-                    T vz[5];
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) vz[k] = v ? zq[c][k].y : zq[c][k].x;
-                    const T *w = ax == 0 ? vx : (ax == 1 ? vy : vz);
-                    T d;
-                    switch (kk[ax]) {
-                    case S_FWD: d = fd_fwd<T>(w[2], w[3], w[4], ih[ax]); break;
-                    case S_BWD: d = fd_bwd<T>(w[2], w[1], w[0], ih[ax]); break;
-                    case S_C2: d = fd_c2<T>(w[3], w[1], ih[ax]); break;
-                    default: d = c4(w[3], w[1], w[4], w[0], ax); break;
-                    }
-                    a[c][ax] = d;
-                }
-            }
-            finish(v, a);
+            if (x + v >= g.nx) continue;
+            T m[3][3];
+            half_of<T>(a, v, m);
+            finish(v, m);
         }
     }
 }
@@ -722,11 +786,9 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                     if constexpr (sizeof(T) == 4) return c4_folded(p1, m1, p2, m2, k1[ax], k2n[ax]);
                     else return fd_c4<T>(p1, m1, p2, m2, ih[ax]);
                 };
-                // Three evaluators: rows and planes inside [2, n-3] of a tile
+                // Two evaluators: rows and planes inside [2, n-3] of a tile
                 // whose columns all lie inside [2, nx-3] use the fourth-order
-                // stencil only; interior rows of a tile that reaches an x end
-                // select the scheme per voxel without branching; rows or
-                // planes on the two outer layers take the general path.
+                // stencil only; the others take stencil_shell.
                 const bool plane_in = ze >= 2 && ze <= g.nz - 3;
                 const bool tile_x_in = x0 >= 2 && x0 + TXW - 1 <= g.nx - 3;
 #pragma unroll
@@ -736,18 +798,17 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                     const int ly = ty + r * TYT + TMA_HY;
                     if (x >= g.nx || y >= g.ny) continue;
                     T epv[2];
-                    // Error terms of voxel v from its Jacobian (finish_j) or
-                    // its Jacobian matrix minus I (finish).
-                    auto finish_j = [&](int v, const T J) {
-                        const T vv = voxel_error<T>(J, jt[r][v], msk[r][v], tol);
+                    // Error terms of a voxel from its Jacobian; returns its e'
+                    // (greedy: its error).
+                    auto finish_j = [&](const T J, const T target, const bool in_mask) -> T {
+                        const T vv = voxel_error<T>(J, target, in_mask, tol);
                         acc_s += (double) vv * (double) vv;
                         const T av = fabs(vv);  // the maximum is exact in the element type
-                        if (msk[r][v] && av > acc_mt) acc_mt = av;
+                        if (in_mask && av > acc_mt) acc_mt = av;
                         T ep = vv;
                         if (!GREEDY && J < delta) ep += zeta * (J - delta);  // src/displacement_field_gradient.c:71-88
-                        epv[v] = ep;
+                        return ep;
                     };
-                    auto finish = [&](int v, const T (&a)[3][3]) { finish_j(v, det_i_plus<T>(a)); };
                     if (row_in && tile_x_in) {
                         if constexpr (sizeof(T) == 4) {
                             // Both voxels at once, as FP32 pairs.
@@ -765,8 +826,8 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                                                      p_splat(k1[2]), p_splat(k2n[2]));
                             }
                             const float2 J2 = det_i_plus2(a);
-                            finish_j(0, J2.x);
-                            finish_j(1, J2.y);
+                            epv[0] = finish_j(J2.x, jt[r][0], msk[r][0]);
+                            epv[1] = finish_j(J2.y, jt[r][1], msk[r][1]);
                         } else {
                             T a0[3][3], a1[3][3];
 #pragma unroll
@@ -782,72 +843,16 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                                 a0[c][2] = c4(zq[r][c][3].x, zq[r][c][1].x, zq[r][c][4].x, zq[r][c][0].x, 2);
                                 a1[c][2] = c4(zq[r][c][3].y, zq[r][c][1].y, zq[r][c][4].y, zq[r][c][0].y, 2);
                             }
-                            finish(0, a0);
-                            finish(1, a1);
-                        }
-                    } else if (row_in) {
-                        // Interior row: the scheme depends on x only
-                        // (src/jacobian.c:113-241): outer column -> one-sided
-                        // in x and second-order central in y, z; penultimate
-                        // column -> second-order central; else fourth order.
-#pragma unroll
-                        for (int v = 0; v < 2; ++v) {
-                            const int xv = x + v;
-                            if (xv >= g.nx) continue;
-                            const bool xo_lo = xv == 0, xo_hi = xv == g.nx - 1;
-                            const bool second = xo_lo || xo_hi || xv == 1 || xv == g.nx - 2;
-                            T a[3][3];
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                const T *p = jp + c * TMA_PLANE + ly * TMA_PX + lx + v;
-                                const T fx = xo_lo ? fd_fwd<T>(p[0], p[1], p[2], ih[0])
-                                                   : (xo_hi ? fd_bwd<T>(p[0], p[-1], p[-2], ih[0])
-                                                            : fd_c2<T>(p[1], p[-1], ih[0]));
-                                const T cx4 = c4(p[1], p[-1], p[2], p[-2], 0);
-                                a[c][0] = second ? fx : cx4;
-                                const T cy4 = c4(p[TMA_PX], p[-TMA_PX], p[2 * TMA_PX], p[-2 * TMA_PX], 1);
-                                const T cy2 = fd_c2<T>(p[TMA_PX], p[-TMA_PX], ih[1]);
-                                a[c][1] = second ? cy2 : cy4;
-                                T zv[5];
-#pragma unroll
-                                for (int k = 0; k < 5; ++k) zv[k] = v ? zq[r][c][k].y : zq[r][c][k].x;
-                                const T cz4 = c4(zv[3], zv[1], zv[4], zv[0], 2);
-                                const T cz2 = fd_c2<T>(zv[3], zv[1], ih[2]);
-                                a[c][2] = second ? cz2 : cz4;
-                            }
-                            finish(v, a);
+                            epv[0] = finish_j(det_i_plus<T>(a0), jt[r][0], msk[r][0]);
+                            epv[1] = finish_j(det_i_plus<T>(a1), jt[r][1], msk[r][1]);
                         }
                     } else {
-#pragma unroll
-                        for (int v = 0; v < 2; ++v) {
-                            const int xv = x + v;
-                            if (xv >= g.nx) continue;
-                            int kk[3];
-                            schemes_at(xv, y, ze, g, kk);
-                            T a[3][3];
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                const T *p = jp + c * TMA_PLANE + ly * TMA_PX + lx + v;
-                                const T vx[5] = {p[-2], p[-1], p[0], p[1], p[2]};
-                                const T vy[5] = {p[-2 * TMA_PX], p[-TMA_PX], p[0], p[TMA_PX], p[2 * TMA_PX]};
-                                T vz[5];
-#pragma unroll
-                                for (int k = 0; k < 5; ++k) vz[k] = v ? zq[r][c][k].y : zq[r][c][k].x;
-#pragma unroll
-                                for (int ax = 0; ax < 3; ++ax) {
-                                    const T *w = ax == 0 ? vx : (ax == 1 ? vy : vz);
-                                    T d;
-                                    switch (kk[ax]) {
-                                    case S_FWD: d = fd_fwd<T>(w[2], w[3], w[4], ih[ax]); break;
-                                    case S_BWD: d = fd_bwd<T>(w[2], w[1], w[0], ih[ax]); break;
-                                    case S_C2: d = fd_c2<T>(w[3], w[1], ih[ax]); break;
-                                    default: d = c4(w[3], w[1], w[4], w[0], ax); break;
-                                    }
-                                    a[c][ax] = d;
-                                }
-                            }
-                            finish(v, a);
-                        }
+                        P2 a[3][3];
+                        stencil_shell<T, TMA_PX, TMA_PLANE>(zq[r], jp + ly * TMA_PX + lx, x, y, ze, g, ih, row_in, a);
+                        const P2 J2 = det_pair_rn<T>(a);
+                        epv[0] = finish_j(J2.x, jt[r][0], msk[r][0]);
+                        epv[1] = T(0);
+                        if (pair_in) epv[1] = finish_j(J2.y, jt[r][1], msk[r][1]);
                     }
                     T *o = ep_out + (qoff - 2 * g.zs) + (long long) y * g.ys + x;
                     if (pair_in)

@@ -153,3 +153,19 @@ def test_any_layout_kernel_keeps_infinities_local(oracle):
         ref = oracle.jacobian(f)
     J = torch_ops.jacobian_raw(torch.from_numpy(f).cuda()).cpu().numpy()
     np.testing.assert_array_equal(np.isfinite(J), np.isfinite(ref))
+
+
+@pytest.mark.parametrize("at", [(4, 5, 3), (2, 2, 2), (8, 10, 15), (5, 1, 12)])
+def test_tma_kernel_keeps_infinities_local(oracle, at):
+    """The same for the TMA kernel: the outer layers share one expression with
+    the fourth-order voxels, which must not read what their scheme does not."""
+    torch = _torch()
+    from disptools_b200 import torch_ops
+    f = np.random.default_rng(4).normal(scale=0.1, size=(3, 9, 11, 16)).astype(np.float32)
+    f[(1,) + at] = np.inf
+    with np.errstate(invalid="ignore"):
+        ref = oracle.jacobian(f.astype(np.float64))
+    J = torch_ops.jacobian_raw(torch.from_numpy(f).cuda()).cpu().numpy()
+    np.testing.assert_array_equal(np.isfinite(J), np.isfinite(ref))
+    ok = np.isfinite(ref)
+    assert np.max(np.abs(J[ok] - ref[ok])) <= 2e-5
