@@ -1066,22 +1066,21 @@ long long queue_time(const std::vector<Geom> &geo, int tile_x, int slots, int bz
     return end;
 }
 
-// Planes per z tile, in [lo, 32], that fill the waves of a persistent grid of
+// Planes per z tile, in [lo, hi], that fill the waves of a persistent grid of
 // `slots` resident blocks: the depth of the shortest launch in queue_time's
-// model, the larger one on ties.  (Deeper tiles cost more than they save: the
-// last ones run alone.  Greedy trial at 256^3: 0.282 ms at 58 planes, 0.274
-// at 32.)  At 256^3 with 32 x 16 tiles and 296 slots this gives 29 planes
-// (1152 tiles, 3.9 waves; 32 planes give 1024 tiles, 3.5 waves).  A
-// volume that does not fill the slots at 32 planes takes thin tiles: a
-// plane costs a block 1.7-2.1 us whether or not its SM has other work, so
-// 40^3 in FP64 is better off as 120 tiles of 6 planes than as 12 of 36
-// (100 iterations: 16.4 -> 4.1 ms).
-int wave_filled_bz(const std::vector<Geom> &geo, int tile_x, int slots, int lo) {
+// model, the larger one on ties.  At 256^3 with 32 x 16 tiles and 296 slots
+// this gives 29 planes up to 32 (1152 tiles, 3.9 waves) and 58 up to 64.
+// Solves that are not tuned stay at 32 or below (greedy trial at 256^3: 248 us
+// at 29 planes, 255 at 32, 249 at 58, 271 at 64).  A volume that does not fill
+// the slots at 32 planes takes thin tiles: a plane costs a block 1.7-2.1 us
+// whether or not its SM has other work, so 40^3 in FP64 is better off as 120
+// tiles of 6 planes than as 12 of 36 (100 iterations: 16.4 -> 4.1 ms).
+int wave_filled_bz(const std::vector<Geom> &geo, int tile_x, int slots, int lo, int hi) {
     int mz = 0;
     for (const Geom &g : geo) mz = std::max(mz, g.nz);
     int best = std::min(mz, 32);
     long long best_t = LLONG_MAX;
-    for (int bz = std::min(32, mz); bz >= std::min(lo, mz); --bz) {
+    for (int bz = std::min(hi, mz); bz >= std::min(lo, mz); --bz) {
         const long long t = queue_time(geo, tile_x, slots, bz, best_t);
         if (t < best_t) {
             best_t = t;
@@ -1092,13 +1091,16 @@ int wave_filled_bz(const std::vector<Geom> &geo, int tile_x, int slots, int lo) 
 }
 
 // Candidate shapes, the one every other must beat by 1 % first: the default
-// x-y shape at `bzw` (the wave-filled depth of the solve, 0: none), which
-// measured 2 % faster than the fixed 32 planes at 256^3 (0.2275 against
-// 0.233 ms a trial), else the fixed default.
-std::vector<TileConfig> tile_candidates(size_t tsize, int bzw) {
+// x-y shape at `bzw` and `bzd` (the wave-filled depths up to 32 and up to 64
+// planes), which measured 2 to 8 % faster than the fixed 32 planes at 256^3
+// (trial 196 us at 32 planes, 185 at 29, 180 at 58; gradient 158, 164, 164),
+// else the fixed default.
+std::vector<TileConfig> tile_candidates(size_t tsize, int bzw, int bzd) {
     std::vector<TileConfig> c;
-    const bool wave = bzw > 0 && bzw != 16 && bzw != 32 && bzw != 64;
+    auto listed = [](int bz) { return bz == 16 || bz == 32 || bz == 64; };
+    const bool wave = !listed(bzw);
     if (wave) c.push_back({32, 16, 16, bzw});
+    if (bzd != bzw && !listed(bzd)) c.push_back({32, 16, 16, bzd});
     const std::vector<TileConfig> fixed = {{32, 16, 16, 32}, {32, 16, 8, 32}, {32, 16, 16, 16}, {32, 16, 16, 64},
                                            {32, 8, 16, 32}};
     c.insert(c.end(), fixed.begin(), fixed.end());
@@ -1131,7 +1133,7 @@ int choose_config(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols, 
         key.mz = std::max(key.mz, v.g.nz);
     }
     if (!gradient || key.voxels < AUTOTUNE_MIN_VOXELS || !autotune_enabled()) {
-        c.bz = wave_filled_bz(geo, 32, slots, 2);
+        c.bz = wave_filled_bz(geo, 32, slots, 2, 32);
         *out = c;
         return DTB_OK;
     }
@@ -1143,7 +1145,8 @@ int choose_config(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols, 
     NvtxRange range("dtb autotune");
     TileConfig best = c;
     float best_ms = FLT_MAX;
-    for (const TileConfig &cand : tile_candidates(sizeof(T), wave_filled_bz(geo, 32, slots, 12))) {
+    for (const TileConfig &cand : tile_candidates(sizeof(T), wave_filled_bz(geo, 32, slots, 12, 32),
+                                                 wave_filled_bz(geo, 32, slots, 12, 64))) {
         float ms = FLT_MAX;
         const int rc = solve_device_on<T>(e, algorithm, vols, p, nullptr, precision, &cand, &ms);
         if (rc != DTB_OK) return rc;

@@ -562,14 +562,13 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
     T *ring = reinterpret_cast<T *>(smem + L::RING_OFF);
     T *vring = reinterpret_cast<T *>(smem + L::VRING_OFF);  // greedy: error-map planes
     __shared__ double red[2 * (NTH / 32)];
-    __shared__ int s_flag, s_fault;
+    __shared__ int s_flag;
     __shared__ T s_dd[3];  // greedy steps of the current tile
 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TPX + tx;
     if (tid == 0) {
         for (int s = 0; s < L::S; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
-        s_fault = 0;
     }
     __syncthreads();
     uint32_t kbase = 0;  // iterations consumed by this block (mbarrier phases)
@@ -682,20 +681,24 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
         if (GREEDY && trial && !stale_zero)
             greedy_prefetch_stale<T, L>(ring + (size_t) ((z0 - 2) & (L::R - 1)) * 3 * TMA_PLANE, tid, NTH, g, x0, y0,
                                         z0 - 2, dst);
+        int stage = (int) (kbase % L::S);  // of iteration `it`, and its barrier's phase
+        uint32_t phase_bit = (kbase / L::S) & 1u;
         for (int it = 0; it < n_it; ++it, qoff += g.zs) {
-            const uint32_t k = kbase + it;
-            const int s = k % L::S;
-            const uint32_t par = (k / L::S) & 1u;
+            const int s = stage;
+            const uint32_t par = phase_bit;
+            if (++stage == L::S) {
+                stage = 0;
+                phase_bit ^= 1u;
+            }
             // Every thread waits for the stage itself (bounded); a timeout is
             // agreed on after the barrier below, so all threads leave together.
             const bool ok = mbar_wait_bounded(&bars[s], par, wait_limit);
-            if (!ok) s_fault = 1;
             const unsigned char *sb = smem + s * L::STAGE_BYTES;
             const int q = z0 - 2 + it, ze = q - 2;
             T *slot = ring + (size_t) (q & (L::R - 1)) * 3 * TMA_PLANE;
             // Candidate plane q (tile + halo): u - eta g, vectorised.
             if (ok) {
-                constexpr int VEC = 16 / (int) sizeof(T);
+                constexpr int VEC = 16 / (int) sizeof(T), RUNS = 3 * TMA_PLANE / VEC;
                 using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
                 const V4 *u4 = reinterpret_cast<const V4 *>(sb);
                 const V4 *g4 = reinterpret_cast<const V4 *>(sb + L::U_BYTES);
@@ -711,7 +714,10 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                 // Counted from the last thread: the runs left over after
                 // whole sweeps go to the last warps, not to warp 0, whose
                 // thread 0 also issues the loads.
-                for (int i = NTH - 1 - tid; i < 3 * TMA_PLANE / VEC; i += NTH) {
+#pragma unroll
+                for (int sweep = 0; sweep < (RUNS + NTH - 1) / NTH; ++sweep) {
+                    const int i = NTH - 1 - tid + sweep * NTH;
+                    if ((sweep + 1) * NTH > RUNS && i >= RUNS) break;
                     V4 a = u4[i];
                     if (trial) {
                         const V4 b = g4[i];
@@ -740,8 +746,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                     msk[r][1] = (m2 >> 8) != 0;
                 }
             }
-            __syncthreads();
-            if (s_fault) {
+            if (__syncthreads_or(!ok)) {
                 failed = true;
                 fail_it = it;
                 break;
@@ -801,13 +806,22 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                     // Error terms of a voxel from its Jacobian; returns its e'
                     // (greedy: its error).
                     auto finish_j = [&](const T J, const T target, const bool in_mask) -> T {
-                        const T vv = voxel_error<T>(J, target, in_mask, tol);
+                        // Without branches (greedy: they cost less, its errors
+                        // are mostly inside the mask or 0).
+                        T vv;
+                        if constexpr (GREEDY) {
+                            vv = voxel_error<T>(J, target, in_mask, tol);
+                        } else {
+                            const T e = J - target, ae = fabs(e);
+                            const T soft = ae < tol ? T(0.0) : copysign(ae - tol, e);
+                            vv = in_mask ? e : soft;
+                        }
                         acc_s += (double) vv * (double) vv;
                         const T av = fabs(vv);  // the maximum is exact in the element type
-                        if (in_mask && av > acc_mt) acc_mt = av;
-                        T ep = vv;
-                        if (!GREEDY && J < delta) ep += zeta * (J - delta);  // src/displacement_field_gradient.c:71-88
-                        return ep;
+                        acc_mt = fmax(acc_mt, in_mask ? av : T(0));
+                        if constexpr (GREEDY) return vv;
+                        const T reg = vv + zeta * (J - delta);  // src/displacement_field_gradient.c:71-88
+                        return J < delta ? reg : vv;
                     };
                     if (row_in && tile_x_in) {
                         if constexpr (sizeof(T) == 4) {
@@ -816,7 +830,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
 #pragma unroll
                             for (int c = 0; c < 3; ++c) {
                                 const T *p = jp + c * TMA_PLANE + ly * TMA_PX + lx;
-                                const float2 xm = ld_pair(p - 2), xc = ld_pair(p), xp = ld_pair(p + 2);
+                                const float2 xm = ld_pair(p - 2), xc = zq[r][c][2], xp = ld_pair(p + 2);
                                 const float2 dx1 = make_float2(__fsub_rn(xc.y, xm.y), __fsub_rn(xp.x, xc.x));
                                 a[c][0] = c4_folded2d(dx1, xp, xm, p_splat(k1[0]), p_splat(k2n[0]));
                                 const float2 ym1 = ld_pair(p - TMA_PX), yp1 = ld_pair(p + TMA_PX);
@@ -925,7 +939,7 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::BAR_OFF);
     T *pxy = reinterpret_cast<T *>(smem + L::P_OFF);
     __shared__ double red[2 * (NTH / 32)];
-    __shared__ int s_flag, s_fault;
+    __shared__ int s_flag;
     // P terms of the x (t = 0..2) and y (t = 3..5) directions.  P column c
     // holds x = x0 + c - 2 (so the own pairs start at even columns), P row r
     // holds y = y0 + r - 1.
@@ -936,7 +950,6 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
     if (tid == 0) {
         for (int s = 0; s < L::S; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
-        s_fault = 0;
     }
     __syncthreads();
     uint32_t kbase = 0;
@@ -987,12 +1000,6 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
             tmap_acquire(tm_e);
             for (int j = 0; j < min(L::S, n_it); ++j) issue(j);
         }
-        auto stage_u = [&](int j) -> const T * {
-            return reinterpret_cast<const T *>(smem + ((kbase + j) % L::S) * L::STAGE_BYTES);
-        };
-        auto stage_e = [&](int j) -> const T * {
-            return reinterpret_cast<const T *>(smem + ((kbase + j) % L::S) * L::STAGE_BYTES + L::U_BYTES);
-        };
 
         const int x = x0 + 2 * tx;       // this thread's columns: x, x + 1
         const int lx = 2 * tx + TMA_HX;  // their box column
@@ -1009,12 +1016,14 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
         bool failed = false;
         int fail_it = 0;
         long long zoff = (long long) (z0 - 4) * g.zs;  // offset of gradient plane z = q - 2
+        // Stages of planes q, q-1, q-2 (counted, not divided for: the remainders
+        // by 5 and 3 were a sixth of the instructions), the barrier's phase of
+        // q, and the P slots of planes p and p-1.
+        int s0 = (int) (kbase % L::S), s1 = 0, s2 = 0;
+        uint32_t phase_bit = (kbase / L::S) & 1u;
+        int ps = 0, ps1 = 0;
         for (int it = 0; it < n_it; ++it, zoff += g.zs) {
-            const uint32_t k = kbase + it;
-            const int s = k % L::S;
-            const uint32_t par = (k / L::S) & 1u;
-            const bool ok = mbar_wait_bounded(&bars[s], par);
-            if (!ok) s_fault = 1;
+            const bool ok = mbar_wait_bounded(&bars[s0], phase_bit);
             const int q = z0 - 2 + it;
             const int p = q - 1;  // plane of P computed now (needs u(q-2..q), e'(q-1))
             P2 pz_new[RYT][3];
@@ -1023,9 +1032,10 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
 #pragma unroll
                 for (int i = 0; i < 3; ++i) pz_new[r][i] = P2{T(0), T(0)};
             if (it >= 2 && ok) {
-                const T *um = stage_u(it - 2), *u0 = stage_u(it - 1), *up = stage_u(it);
-                const T *e0 = stage_e(it - 1);
-                const int ps = ring_slot(p, L::NP);
+                const T *um = reinterpret_cast<const T *>(smem + s2 * L::STAGE_BYTES);
+                const T *u0 = reinterpret_cast<const T *>(smem + s1 * L::STAGE_BYTES);
+                const T *up = reinterpret_cast<const T *>(smem + s0 * L::STAGE_BYTES);
+                const T *e0 = reinterpret_cast<const T *>(smem + s1 * L::STAGE_BYTES + L::U_BYTES);
                 // FP32 states every rounding, so the scalar (halo) and the
                 // paired (own) cells give the same bits: a minor is a
                 // difference of two products, a diagonal entry d h + 1 one
@@ -1164,8 +1174,7 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
                     }
                 }
             }
-            __syncthreads();
-            if (s_fault) {
+            if (__syncthreads_or(!ok)) {
                 failed = true;
                 fail_it = it;
                 break;
@@ -1173,7 +1182,6 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
             if (tid == 0 && it >= 2 && it - 2 + L::S < n_it) issue(it - 2 + L::S);
             const int z = q - 2;  // gradient plane: P(z-1), P(z), P(z+1) ready
             if (own && it >= 3 && z >= z0 && z < z1 && z >= 1 && z < g.nz - 1 && x < g.nx - 1 && x + 1 >= 1) {
-                const int ps = ring_slot(z, L::NP);
                 const bool in0 = x >= 1, in1 = x + 1 < g.nx - 1;
 #pragma unroll
                 for (int r = 0; r < RYT; ++r) {
@@ -1187,11 +1195,11 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
                         float2 t[3][3];
 #pragma unroll
                         for (int i = 0; i < 3; ++i) {
-                            const float2 a = ld_pair(PT(ps, i, rp, cp - 2)), b = ld_pair(PT(ps, i, rp, cp)),
-                                         c = ld_pair(PT(ps, i, rp, cp + 2));
+                            const float2 a = ld_pair(PT(ps1, i, rp, cp - 2)), b = ld_pair(PT(ps1, i, rp, cp)),
+                                         c = ld_pair(PT(ps1, i, rp, cp + 2));
                             t[i][0] = p_mul(p_splat(ihx), make_float2(__fsub_rn(a.y, b.y), __fsub_rn(b.x, c.x)));
-                            const float2 ym = ld_pair(PT(ps, 3 + i, rp - 1, cp)),
-                                         yp = ld_pair(PT(ps, 3 + i, rp + 1, cp));
+                            const float2 ym = ld_pair(PT(ps1, 3 + i, rp - 1, cp)),
+                                         yp = ld_pair(PT(ps1, 3 + i, rp + 1, cp));
                             t[i][1] = p_mul(p_splat(ihy), p_sub(ym, yp));
                             t[i][2] = p_mul(p_splat(ihz), p_sub(pz_m2[r][i], pz_new[r][i]));
                         }
@@ -1204,12 +1212,12 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
                         T t[2][3][3];
 #pragma unroll
                         for (int i = 0; i < 3; ++i) {
-                            const auto a = ld_pair(PT(ps, i, rp, cp - 2)), b = ld_pair(PT(ps, i, rp, cp)),
-                                       c = ld_pair(PT(ps, i, rp, cp + 2));
+                            const auto a = ld_pair(PT(ps1, i, rp, cp - 2)), b = ld_pair(PT(ps1, i, rp, cp)),
+                                       c = ld_pair(PT(ps1, i, rp, cp + 2));
                             t[0][i][0] = ihx * (a.y - b.y);
                             t[1][i][0] = ihx * (b.x - c.x);
-                            const auto ym = ld_pair(PT(ps, 3 + i, rp - 1, cp)),
-                                       yp = ld_pair(PT(ps, 3 + i, rp + 1, cp));
+                            const auto ym = ld_pair(PT(ps1, 3 + i, rp - 1, cp)),
+                                       yp = ld_pair(PT(ps1, 3 + i, rp + 1, cp));
                             t[0][i][1] = ihy * (ym.x - yp.x);
                             t[1][i][1] = ihy * (ym.y - yp.y);
                             t[0][i][2] = ihz * (pz_m2[r][i].x - pz_new[r][i].x);
@@ -1253,6 +1261,14 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
                     pz_m2[r][i] = pz_m1[r][i];
                     pz_m1[r][i] = pz_new[r][i];
                 }
+            s2 = s1;
+            s1 = s0;
+            if (++s0 == L::S) {
+                s0 = 0;
+                phase_bit ^= 1u;
+            }
+            ps1 = ps;
+            ps = ps + 1 < L::NP ? ps + 1 : 0;
         }
         if (failed) {
             if (tid == 0) tma_fault<L::S>(st, bars, kbase, fail_it + 1, issued_n);
