@@ -585,10 +585,11 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
         need += align(N * sizeof(T)) + align(N);     // target map, mask
         need += 2 * align(N * sizeof(T));            // e' (gradient) or error maps (greedy)
         need += align(t * sizeof(double2)) + align(t * sizeof(double));
-        need += align(sizeof(SolverState)) + align(7 * sizeof(CUtensorMap));
+        need += align(7 * sizeof(CUtensorMap));
         need += align((size_t) log_cap * sizeof(IterLog));
     }
-    need += align(count * sizeof(VolumeDesc<T>)) + align(total_tiles * sizeof(int)) + align(2 * sizeof(TileQueue));
+    need += align(count * sizeof(VolumeDesc<T>)) + align(total_tiles * sizeof(int)) + align(2 * sizeof(TileQueue)) +
+            align(count * sizeof(SolverState));
 
     char *base = nullptr;
     int rc = workspace(need, &base);
@@ -599,6 +600,7 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
     std::vector<SolverState> hst(count);
     std::vector<int> tile_vol(total_tiles);
     std::vector<CUtensorMap *> d_maps(count);
+    SolverState *d_state0 = cv.take<SolverState>(count);
     for (int i = 0; i < count; ++i) {
         const Geom &g = geo[i];
         const Geom &gu = vols[i].g;  // caller's dense layout
@@ -623,7 +625,7 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
         }
         d.part_t = cv.take<double2>(tiles[i]);
         d.part_g = cv.take<double>(tiles[i]);
-        d.st = cv.take<SolverState>(1);
+        d.st = d_state0 + i;
         IterLog *log = log_cap ? cv.take<IterLog>((size_t) log_cap) : nullptr;
         d_maps[i] = cv.take<CUtensorMap>(7);
         const int bz = bz_for(g.nz, cfg.bz);
@@ -749,16 +751,17 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
                                        : trial_tma_blocks_per_sm<T>(tile_x, trial_ty));
     const int grid_t = std::min(total_tiles, std::max(1, bps_t) * num_sms());
     const int grid_g = std::min(total_tiles, std::max(1, gradient_tma_blocks_per_sm<T>(tile_x, threads_y)) * num_sms());
+    const int *tv = count > 1 ? d_tile_vol : nullptr;
     auto launch_t = [&](unsigned char *flag) -> cudaError_t {
         if (rel)
             return launch_trial_rel<T>(d_desc, d_tile_vol, total_tiles, grid_t, stream, flag, tile_x, trial_ty,
                                        d_queues);
-        if (gradient) return launch_trial_tma<T>(d_desc, d_tile_vol, total_tiles, grid_t, stream, flag, tile_x, trial_ty,
-                                                    d_queues, cfg.pf);
-        return launch_greedy_tma<T>(d_desc, d_tile_vol, total_tiles, grid_t, stream, flag, d_queues);
+        if (gradient) return launch_trial_tma<T>(d_desc, tv, d_state0, total_tiles, grid_t, stream, flag, tile_x,
+                                                 trial_ty, d_queues, cfg.pf);
+        return launch_greedy_tma<T>(d_desc, tv, d_state0, total_tiles, grid_t, stream, flag, d_queues);
     };
     auto launch_g = [&](unsigned char *flag) -> cudaError_t {
-        return launch_gradient_tma<T>(d_desc, d_tile_vol, total_tiles, grid_g, stream, flag, tile_x, threads_y,
+        return launch_gradient_tma<T>(d_desc, tv, d_state0, total_tiles, grid_g, stream, flag, tile_x, threads_y,
                                       d_queues + 1, cfg.pf);
     };
 

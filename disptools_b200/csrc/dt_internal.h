@@ -124,15 +124,17 @@ struct VolumeDesc {
 // Launch wrappers, instantiated for float and double in dt_kernels_*.cu.
 // `work_flag` (may be null) is set to 1 by a launch that did work for at
 // least one volume (profiling separates real launches from no-op ones).
+// `tile_vol` maps tiles to volumes (null: one volume) and `states` is their
+// state array.
 // TMA kernels of the gradient method; tiles are tile_x (64 or 32) by TT_Y
 // voxels; threads_y rows of threads (8 or 16).  `pf` > 0 prefetches into L2
 // the boxes of the plane pf iterations ahead of each load.
 template <typename T>
-cudaError_t launch_trial_tma(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_trial_tma(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                              cudaStream_t s, unsigned char *work_flag, int tile_x, int threads_y, TileQueue *queue,
                              int pf);
 template <typename T>
-cudaError_t launch_gradient_tma(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_gradient_tma(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                                 cudaStream_t s, unsigned char *work_flag, int tile_x, int threads_y,
                                 TileQueue *queue, int pf);
 template <typename T>
@@ -149,7 +151,7 @@ template <typename T>
 int gradient_tma_blocks_per_sm(int tile_x, int threads_y);
 // TMA trial kernel of the greedy method (tiles 32 x TT_Y).
 template <typename T>
-cudaError_t launch_greedy_tma(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_greedy_tma(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                               cudaStream_t s, unsigned char *work_flag, TileQueue *queue);
 template <typename T>
 int greedy_tma_blocks_per_sm();

@@ -119,14 +119,15 @@ struct GradTmaLayout {
 };
 
 // Takes the next tile of a persistent launch (-1 when none is left; the
-// block is then counted out and the last one resets the queue).  BDX is the
+// block is then counted out and the last one resets the queue).  A block's
+// first tile is its own number, without the queue's round trip.  BDX is the
 // block's x dimension.
 template <int BDX>
 __device__ __forceinline__ int take_tile(TileQueue *q, int total, int *s_tile) {
     const int tid = threadIdx.y * BDX + threadIdx.x;
     __syncthreads();  // everyone has read the previous s_tile
     if (tid == 0) {
-        int t = (int) atomicAdd(&q->next, 1u);
+        int t = (int) (gridDim.x + atomicAdd(&q->next, 1u));
         if (t >= total) {
             t = -1;
             __threadfence();
@@ -549,8 +550,8 @@ __device__ __forceinline__ void stencil_pair(const typename PairOf<T>::type (&zq
 // content of the new field buffer, and the stored map is the error itself.
 template <typename T, int TXW, int TYT, bool GREEDY = false>
 __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof(T) == 4) ? 2 : 1)
-    k_trial_tma(const VolumeDesc<T> *__restrict__ vols, const int *__restrict__ tile_vol, int total_tiles,
-                unsigned char *__restrict__ work_flag, TileQueue *queue, int pf) {
+    k_trial_tma(const VolumeDesc<T> *__restrict__ vols, const int *__restrict__ tile_vol, SolverState *states,
+                int total_tiles, unsigned char *__restrict__ work_flag, TileQueue *queue, int pf) {
     using L = TrialTmaLayout<T, TXW, GREEDY>;
     constexpr int TPX = TXW / 2, NTH = TPX * TYT, RYT = TT_Y / TYT;
     constexpr int TMA_PX = L::TMA_PX, TMA_PLANE = L::TMA_PLANE;
@@ -562,6 +563,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
     T *ring = reinterpret_cast<T *>(smem + L::RING_OFF);
     T *vring = reinterpret_cast<T *>(smem + L::VRING_OFF);  // greedy: error-map planes
     __shared__ double red[2 * (NTH / 32)];
+    __shared__ unsigned long long s_words[sizeof(SolverState) / 8];
     __shared__ int s_flag;
     __shared__ T s_dd[3];  // greedy steps of the current tile
 
@@ -575,19 +577,21 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
     uint32_t vbase = 0;  // greedy: error-map planes loaded by this block (ring position)
 
     __shared__ int s_tile;
-    for (int tile = take_tile<TPX>(queue, total_tiles, &s_tile); tile >= 0;
+    for (int tile = (int) blockIdx.x; tile >= 0;
          tile = take_tile<TPX>(queue, total_tiles, &s_tile)) {
-        const VolumeDesc<T> &V = vols[tile_vol[tile]];
-        SolverState *st = V.st;
-        if (ldcg_int(&st->done)) continue;
+        const int vol = tile_vol ? tile_vol[tile] : 0;
+        const VolumeDesc<T> &V = vols[vol];
+        SolverState *st = states + vol;
+        // All at once: a launch on a small volume is a chain of such waits.
         const Geom g = V.g;
-        const int phase = ldcg_int(&st->phase);
-        const int old_b = ldcg_int(&st->old_buf);
+        const int done = ldcg_int(&st->done), phase = ldcg_int(&st->phase), old_b = ldcg_int(&st->old_buf);
         const int v_cur = GREEDY ? ldcg_int(&st->v_cur) : 0;
         // Greedy: the new buffer's boundary values are all +0 when it is
         // buffer 1 or the initial field's boundary is; no copies then.
         const bool stale_zero = GREEDY && (old_b == 0 || !ldcg_int(&st->b0_nonzero));
         const double eta = __ldcg(&st->eta);
+        const T tol = (T) st->tolerance, delta = (T) st->delta, zeta = (T) st->zeta;
+        if (done) continue;
         const bool trial = phase != PH_EVAL0;
         const int lt = tile - V.tile_begin;
         const int txi = lt % V.tiles_x, tyi = (lt / V.tiles_x) % V.tiles_y, tzi = lt / (V.tiles_x * V.tiles_y);
@@ -606,7 +610,6 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
             __syncthreads();
         }
         const T ih[3] = {(T) g.ih[0], (T) g.ih[1], (T) g.ih[2]};
-        const T tol = (T) st->tolerance, delta = (T) st->delta, zeta = (T) st->zeta;
 
         int issued_n = 0;  // iterations whose loads were issued (thread 0)
         const unsigned wait_limit = V.wait_limit ? V.wait_limit : (1u << 22);
@@ -896,13 +899,21 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                 ssum += pp.x;
                 smax = fmax(smax, pp.y);
             }
+            // The step control works on a copy that the block fetches and
+            // returns at once, not on one field after the other.
+            static_assert(sizeof(SolverState) % 8 == 0 && sizeof(SolverState) / 8 <= NTH, "one word a thread");
+            unsigned long long *gst = reinterpret_cast<unsigned long long *>(st);
+            if (tid < (int) sizeof(SolverState) / 8) s_words[tid] = __ldcg(gst + tid);
             const double2 tot = block_reduce_n<NTH, TPX>(ssum, smax, red);
             if (tid == 0) {
-                st->ticket_t = 0;
-                control_after_trial(st, tot.x, tot.y);
+                SolverState *now = reinterpret_cast<SolverState *>(s_words);
+                now->ticket_t = 0;
+                control_after_trial(now, tot.x, tot.y);
                 if (work_flag) *work_flag = 1;
-                __threadfence();
             }
+            __syncthreads();
+            if (tid < (int) sizeof(SolverState) / 8) gst[tid] = s_words[tid];
+            __threadfence();
         }
         __syncthreads();
     }
@@ -923,8 +934,8 @@ __host__ __device__ constexpr int grad_halo_rows() {
 // FP32 (shared memory allows no more), one for FP64.
 template <typename T, int TXW, int TYT>
 __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeof(T) == 4 ? 2 : 1)
-    k_gradient_tma(const VolumeDesc<T> *__restrict__ vols, const int *__restrict__ tile_vol, int total_tiles,
-                   unsigned char *__restrict__ work_flag, TileQueue *queue, int pf) {
+    k_gradient_tma(const VolumeDesc<T> *__restrict__ vols, const int *__restrict__ tile_vol, SolverState *states,
+                   int total_tiles, unsigned char *__restrict__ work_flag, TileQueue *queue, int pf) {
     using L = GradTmaLayout<T, TXW>;
     constexpr int TPX = TXW / 2, RYT = TT_Y / TYT;
     constexpr int NHALO = 2 * TT_Y + TXW;  // halo tasks: x sides (one cell each), y sides (two cells each)
@@ -955,13 +966,14 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
     uint32_t kbase = 0;
 
     __shared__ int s_tile;
-    for (int tile = take_tile<TPX>(queue, total_tiles, &s_tile); tile >= 0;
+    for (int tile = (int) blockIdx.x; tile >= 0;
          tile = take_tile<TPX>(queue, total_tiles, &s_tile)) {
-        const VolumeDesc<T> &V = vols[tile_vol[tile]];
-        SolverState *st = V.st;
-        if (ldcg_int(&st->done) || !ldcg_int(&st->need_gradient)) continue;
+        const int vol = tile_vol ? tile_vol[tile] : 0;
+        const VolumeDesc<T> &V = vols[vol];
+        SolverState *st = states + vol;
         const Geom g = V.g;
-        const int old_b = ldcg_int(&st->old_buf);
+        const int done = ldcg_int(&st->done), wanted = ldcg_int(&st->need_gradient), old_b = ldcg_int(&st->old_buf);
+        if (done || !wanted) continue;
         const int lt = tile - V.tile_begin;
         const int txi = lt % V.tiles_x, tyi = (lt / V.tiles_x) % V.tiles_y, tzi = lt / (V.tiles_x * V.tiles_y);
         const int x0 = txi * TXW, y0 = tyi * TT_Y, z0 = tzi * V.bz;
@@ -1396,7 +1408,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
     // registers, which the plane loop needs): inverse spacing, the wait bound.
     __shared__ T s_ih[3];
     __shared__ unsigned s_wait;
-    for (int tile = take_tile<TPX>(queue, total_tiles, &s_tile); tile >= 0;
+    for (int tile = (int) blockIdx.x; tile >= 0;
          tile = take_tile<TPX>(queue, total_tiles, &s_tile)) {
         const VolumeDesc<T> &V = vols[tile_vol[tile]];
         SolverState *st = V.st;
@@ -1752,40 +1764,40 @@ int trial_rel_blocks_v() {
 }
 
 template <typename T, int TXW, int TYT>
-cudaError_t launch_trial_tma_v(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_trial_tma_v(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                                cudaStream_t s, unsigned char *work_flag, TileQueue *queue, int pf) {
     constexpr int smem = TrialTmaLayout<T, TXW>::BYTES + 128;
     static std::atomic<unsigned long long> devs{0};
     const cudaError_t attr = opt_in_smem(k_trial_tma<T, TXW, TYT>, smem, devs);
     if (attr != cudaSuccess) return attr;
-    k_trial_tma<T, TXW, TYT><<<grid, dim3(TXW / 2, TYT), smem, s>>>(vols, tile_vol, total_tiles, work_flag, queue,
-                                                                     pf);
+    k_trial_tma<T, TXW, TYT><<<grid, dim3(TXW / 2, TYT), smem, s>>>(vols, tile_vol, states, total_tiles, work_flag,
+                                                                     queue, pf);
     count_launch();
     return cudaGetLastError();
 }
 
 template <typename T, int TXW, int TYT>
-cudaError_t launch_greedy_tma_v(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_greedy_tma_v(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                                 cudaStream_t s, unsigned char *work_flag, TileQueue *queue) {
     constexpr int smem = TrialTmaLayout<T, TXW, true>::BYTES + 128;
     static std::atomic<unsigned long long> devs{0};
     const cudaError_t attr = opt_in_smem(k_trial_tma<T, TXW, TYT, true>, smem, devs);
     if (attr != cudaSuccess) return attr;
-    k_trial_tma<T, TXW, TYT, true><<<grid, dim3(TXW / 2, TYT), smem, s>>>(vols, tile_vol, total_tiles, work_flag,
-                                                                           queue, 0);
+    k_trial_tma<T, TXW, TYT, true><<<grid, dim3(TXW / 2, TYT), smem, s>>>(vols, tile_vol, states, total_tiles,
+                                                                           work_flag, queue, 0);
     count_launch();
     return cudaGetLastError();
 }
 
 template <typename T, int TXW, int TYT>
-cudaError_t launch_gradient_tma_v(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_gradient_tma_v(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                                   cudaStream_t s, unsigned char *work_flag, TileQueue *queue, int pf) {
     constexpr int smem = GradTmaLayout<T, TXW>::BYTES + 128;
     static std::atomic<unsigned long long> devs{0};
     const cudaError_t attr = opt_in_smem(k_gradient_tma<T, TXW, TYT>, smem, devs);
     if (attr != cudaSuccess) return attr;
     k_gradient_tma<T, TXW, TYT><<<grid, dim3(TXW / 2, TYT + grad_halo_rows<TXW>()), smem, s>>>(
-        vols, tile_vol, total_tiles, work_flag, queue, pf);
+        vols, tile_vol, states, total_tiles, work_flag, queue, pf);
     count_launch();
     return cudaGetLastError();
 }
@@ -1839,14 +1851,14 @@ int gradient_blocks_v() {
 //   tile_x 32, threads_y 8   128 threads of two rows
 //   tile_x 64, threads_y 8   FP32 only, 256 threads of two rows
 template <typename T>
-cudaError_t launch_trial_tma(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_trial_tma(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                              cudaStream_t s, unsigned char *work_flag, int tile_x, int threads_y, TileQueue *q,
                              int pf) {
     if constexpr (sizeof(T) == 4)
         if (tile_x == 64)
-            return launch_trial_tma_v<T, 64, 16>(vols, tile_vol, total_tiles, grid, s, work_flag, q, pf);
-    if (threads_y == 8) return launch_trial_tma_v<T, 32, 8>(vols, tile_vol, total_tiles, grid, s, work_flag, q, pf);
-    return launch_trial_tma_v<T, 32, 16>(vols, tile_vol, total_tiles, grid, s, work_flag, q, pf);
+            return launch_trial_tma_v<T, 64, 16>(vols, tile_vol, states, total_tiles, grid, s, work_flag, q, pf);
+    if (threads_y == 8) return launch_trial_tma_v<T, 32, 8>(vols, tile_vol, states, total_tiles, grid, s, work_flag, q, pf);
+    return launch_trial_tma_v<T, 32, 16>(vols, tile_vol, states, total_tiles, grid, s, work_flag, q, pf);
 }
 
 // Trial kernel without the per-plane barrier (same tile shapes as
@@ -1868,22 +1880,22 @@ int trial_rel_blocks_per_sm(int tile_x, int threads_y) {
 }
 
 template <typename T>
-cudaError_t launch_gradient_tma(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_gradient_tma(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                                 cudaStream_t s, unsigned char *work_flag, int tile_x, int threads_y, TileQueue *q,
                                 int pf) {
     if constexpr (sizeof(T) == 4)
         if (tile_x == 64)
-            return launch_gradient_tma_v<T, 64, 8>(vols, tile_vol, total_tiles, grid, s, work_flag, q, pf);
+            return launch_gradient_tma_v<T, 64, 8>(vols, tile_vol, states, total_tiles, grid, s, work_flag, q, pf);
     if (threads_y == 16)
-        return launch_gradient_tma_v<T, 32, 16>(vols, tile_vol, total_tiles, grid, s, work_flag, q, pf);
-    return launch_gradient_tma_v<T, 32, 8>(vols, tile_vol, total_tiles, grid, s, work_flag, q, pf);
+        return launch_gradient_tma_v<T, 32, 16>(vols, tile_vol, states, total_tiles, grid, s, work_flag, q, pf);
+    return launch_gradient_tma_v<T, 32, 8>(vols, tile_vol, states, total_tiles, grid, s, work_flag, q, pf);
 }
 
 // Greedy trial: tile 32 x TT_Y, 16 x 16 threads.
 template <typename T>
-cudaError_t launch_greedy_tma(const VolumeDesc<T> *vols, const int *tile_vol, int total_tiles, int grid,
+cudaError_t launch_greedy_tma(const VolumeDesc<T> *vols, const int *tile_vol, SolverState *states, int total_tiles, int grid,
                               cudaStream_t s, unsigned char *work_flag, TileQueue *q) {
-    return launch_greedy_tma_v<T, 32, 16>(vols, tile_vol, total_tiles, grid, s, work_flag, q);
+    return launch_greedy_tma_v<T, 32, 16>(vols, tile_vol, states, total_tiles, grid, s, work_flag, q);
 }
 template <typename T>
 int greedy_tma_blocks_per_sm() {
@@ -3276,12 +3288,15 @@ cudaError_t launch_adjoint_tma(const CUtensorMap &tm_u, const Geom &g, const T *
 }
 
 #define DTB_INSTANTIATE_TMA(T)                                                                              \
-    template cudaError_t launch_trial_tma<T>(const VolumeDesc<T> *, const int *, int, int, cudaStream_t,    \
+    template cudaError_t launch_trial_tma<T>(const VolumeDesc<T> *, const int *, SolverState *, int, int,     \
+                                             cudaStream_t, \
                                              unsigned char *, int, int, TileQueue *, int);                  \
-    template cudaError_t launch_gradient_tma<T>(const VolumeDesc<T> *, const int *, int, int, cudaStream_t, \
+    template cudaError_t launch_gradient_tma<T>(const VolumeDesc<T> *, const int *, SolverState *, int, int,  \
+                                                cudaStream_t, \
                                                 unsigned char *, int, int, TileQueue *, int);               \
     template int trial_tma_blocks_per_sm<T>(int, int);                                                      \
-    template cudaError_t launch_greedy_tma<T>(const VolumeDesc<T> *, const int *, int, int, cudaStream_t,   \
+    template cudaError_t launch_greedy_tma<T>(const VolumeDesc<T> *, const int *, SolverState *, int, int,    \
+                                              cudaStream_t, \
                                               unsigned char *, TileQueue *);                                \
     template int greedy_tma_blocks_per_sm<T>();                                                             \
     template cudaError_t launch_jacobian_tma<T>(const CUtensorMap &, const Geom &, T *, long long, long long, int, \
