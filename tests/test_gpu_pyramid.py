@@ -53,6 +53,22 @@ def test_resample_bitwise(dtype, nearest, src, dst):
     np.testing.assert_array_equal(got, P.resample(v, dst, nearest))
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nearest", [False, True])
+@pytest.mark.parametrize("src,dst", [
+    ((5, 3, 40), (16, 8, 32)),
+    ((20, 9, 33), (33, 17, 65)),
+    ((40, 19, 70), (17, 9, 33)),
+    ((1, 1, 1), (15, 7, 31)),
+    ((3, 2, 2), (130, 1, 1)),
+    ((50, 40, 3), (49, 41, 100)),
+])
+def test_resample_tile_edges(dtype, nearest, src, dst):
+    v = np.random.default_rng(9).standard_normal((2,) + src).astype(dtype)
+    got = D.resample(torch.from_numpy(v).cuda(), dst, nearest).cpu().numpy()
+    np.testing.assert_array_equal(got, P.resample(v, dst, nearest))
+
+
 def test_scale_image_anisotropic_bitwise():
     v = np.random.default_rng(3).standard_normal((1, 20, 24, 18))
     sp = (0.8, 1.25, 2.0)
