@@ -32,8 +32,9 @@ namespace dtb {
 constexpr int JA_X = BX, JA_Y = BY, JA_NT = JA_X * JA_Y;
 constexpr int JA_PX = JA_X + 4, JA_PY = JA_Y + 4, JA_ROWS = 3 * JA_PY, JA_PLANE = JA_ROWS * JA_PX;
 constexpr int JA_D = 3, JA_NS = JA_D + 3;
-// Copies: 252 threads take 36 columns of 7 rows at a time.
-constexpr int JA_RG = JA_NT / JA_PX, JA_SWEEPS = (JA_ROWS + JA_RG - 1) / JA_RG;
+// Copies: 216 threads take the 36 columns of 6 rows at a time, two sweeps a component.
+constexpr int JA_RG = JA_PY / 2;
+static_assert(JA_RG * JA_PX <= JA_NT);
 
 // Resident blocks per SM: 32 warps at 64 registers (FP32), 16 at 128 (FP64).
 template <typename T>
@@ -56,13 +57,6 @@ struct JacOut {
     int first = 0, last = 0;  // the last writes exp(scale * sum) instead
 };
 
-// Copies BYTES bytes to shared memory, zeros when !ok.
-template <int BYTES>
-__device__ __forceinline__ void cp_async_or_zero(void *dst_smem, const void *src, bool ok) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(dst_smem)), "l"(src), "n"(BYTES),
-                 "r"(ok ? BYTES : 0)
-                 : "memory");
-}
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
@@ -96,22 +90,27 @@ struct CentralWeights {
 
 // The stencil matrix of a voxel: `p` its element of the centre plane's box,
 // zq its column's values of planes ze-2 .. ze+2.  A warp is one row of the
-// tile, so `deep` (all its voxels take fourth-order differences) is uniform.
-// Other voxels take fourth-order differences where `c4`, and are second order
-// along every axis elsewhere (schemes_at), one-sided where they lie on a face.
+// tile, so `deep` (all its voxels take fourth-order differences) is uniform
+// and has code without a choice per voxel.  Other voxels take fourth-order
+// differences where `c4`, and are second order along every axis elsewhere
+// (schemes_at), one-sided where they lie on a face.
 template <typename TI, typename T>
 __device__ __forceinline__ void stencil_voxel(const TI *p, const TI (&zq)[3][5], int x, int y, int z, const Geom &g,
                                               const T (&ih)[3], bool deep, bool c4, T (&a)[3][3]) {
-    const CentralWeights<T> w(ih, deep || c4);
+    auto central = [&](const CentralWeights<T> &w, auto second) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const TI *q = p + c * JA_PY * JA_PX;
-        const T xd2 = (T) q[2] - (T) q[-2], yd2 = (T) q[2 * JA_PX] - (T) q[-2 * JA_PX], zd2 = (T) zq[c][4] - (T) zq[c][0];
-        a[c][0] = w((T) q[1] - (T) q[-1], deep || c4 ? xd2 : T(0), 0);
-        a[c][1] = w((T) q[JA_PX] - (T) q[-JA_PX], deep || c4 ? yd2 : T(0), 1);
-        a[c][2] = w((T) zq[c][3] - (T) zq[c][1], deep || c4 ? zd2 : T(0), 2);
+        for (int c = 0; c < 3; ++c) {
+            const TI *q = p + c * JA_PY * JA_PX;
+            a[c][0] = w((T) q[1] - (T) q[-1], second((T) q[2] - (T) q[-2]), 0);
+            a[c][1] = w((T) q[JA_PX] - (T) q[-JA_PX], second((T) q[2 * JA_PX] - (T) q[-2 * JA_PX]), 1);
+            a[c][2] = w((T) zq[c][3] - (T) zq[c][1], second((T) zq[c][4] - (T) zq[c][0]), 2);
+        }
+    };
+    if (deep) {
+        central(CentralWeights<T>(ih, true), [](T d2) { return d2; });
+        return;
     }
-    if (deep) return;
+    central(CentralWeights<T>(ih, c4), [&](T d2) { return c4 ? d2 : T(0); });
     if (x == 0) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -155,34 +154,39 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
     k_jacobian_async(const TI *__restrict__ field, const Geom g, const JacOut<T> out, int bz) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TI *ring = reinterpret_cast<TI *>(smem_raw);
-    __shared__ long long s_row[JA_ROWS];  // start of each box row in plane 0, -1 outside the volume
     const int tid = threadIdx.x, tx = tid % JA_X, ty = tid / JA_X;
     const int tiles_x = (g.nx + JA_X - 1) / JA_X, tiles_y = (g.ny + JA_Y - 1) / JA_Y;
     const int txy = (int) blockIdx.x / tiles_x;
     const int x0 = ((int) blockIdx.x - txy * tiles_x) * JA_X, y0 = (txy % tiles_y) * JA_Y, z0 = (txy / tiles_y) * bz;
     const int z1 = min(z0 + bz, g.nz);
-    if (tid < JA_ROWS) {
-        const int c = tid / JA_PY, gy = y0 - 2 + tid % JA_PY;
-        s_row[tid] = gy >= 0 && gy < g.ny ? c * g.cs + gy * g.ys : -1;
+    // Box positions outside the volume stay zero: their x and y are the same
+    // in every plane, planes below it are never copied, planes above it are
+    // cleared.
+    if (z0 < 2 || y0 < 2 || x0 < 2 || y0 + JA_Y + 2 > g.ny || x0 + JA_X + 2 > g.nx) {
+        for (int i = tid; i < JA_NS * JA_PLANE; i += JA_NT) ring[i] = TI(0);
+        __syncthreads();
     }
-    __syncthreads();
-    const int col = tid % JA_PX, rg = tid / JA_PX;
-    const int gx = x0 - 2 + col;
-    const bool copies = tid < JA_RG * JA_PX, col_ok = gx >= 0 && gx < g.nx;
+    const int rg = tid / JA_PX, col = tid - rg * JA_PX;
+    const int gx = x0 - 2 + col, gy = y0 - 2 + rg;
+    const bool col_ok = rg < JA_RG && gx >= 0 && gx < g.nx;
+    const bool lo = col_ok && gy >= 0 && gy < g.ny, hi = col_ok && gy + JA_RG >= 0 && gy + JA_RG < g.ny;
+    const TI *src = field + ((z0 - 2) * g.zs + gy * g.ys + gx);  // in the next plane to copy
     // Copies plane zp (tile and halo) into its slot; always one group.
     auto load_plane = [&](int zp, int slot) {
-        if (copies && zp <= z1 + 1) {
-            TI *dst = ring + slot * JA_PLANE + rg * JA_PX + col;
-            const bool ok = col_ok && zp >= 0 && zp < g.nz;
-            const TI *src = field + (zp * g.zs + gx);
+        if (zp >= 0 && zp <= z1 + 1) {
+            TI *dst = ring + slot * JA_PLANE + tid;
+            if (zp < g.nz) {
+                const TI *up = src + JA_RG * g.ys;
 #pragma unroll
-            for (int k = 0; k < JA_SWEEPS; ++k) {
-                if ((k + 1) * JA_RG > JA_ROWS && rg + k * JA_RG >= JA_ROWS) break;
-                const long long r = s_row[rg + k * JA_RG];
-                const bool in = ok && r >= 0;
-                cp_async_or_zero<(int) sizeof(TI)>(dst + k * JA_RG * JA_PX, in ? src + r : field, in);
+                for (int c = 0; c < 3; ++c) {
+                    if (lo) cp_async_elem<(int) sizeof(TI)>(dst + c * JA_PY * JA_PX, src + c * g.cs);
+                    if (hi) cp_async_elem<(int) sizeof(TI)>(dst + (c * JA_PY + JA_RG) * JA_PX, up + c * g.cs);
+                }
+            } else {
+                for (int i = tid; i < JA_PLANE; i += JA_NT) ring[slot * JA_PLANE + i] = TI(0);
             }
         }
+        src += g.zs;
         cp_async_commit();
     };
     for (int j = 0; j < JA_D; ++j) load_plane(z0 - 2 + j, j);
@@ -254,17 +258,19 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
     cp_async_wait_all();
 }
 
-// Planes per block: thin tiles where the volume does not fill the device.  A
-// block of bz planes takes bz + 4 plane-times and about two more to start;
-// below one wave of blocks the launch lasts that long, above it the blocks
-// backfill and half a block is left over at the end.
-inline int jacobian_depth(const Geom &g, int slots) {
-    const double cols = (double) ((g.nx + JA_X - 1) / JA_X) * ((g.ny + JA_Y - 1) / JA_Y);
+// Planes per block.  A block of bz planes takes bz + 4 plane-times and about
+// two more to start; blocks run in waves of `slots`, of which the last is
+// shorter where it leaves the SMs fewer than their `resident` blocks (a block
+// alone on an SM runs faster, though not in proportion).
+inline int jacobian_depth(const Geom &g, int resident, int num_sms) {
+    const long long cols = (long long) ((g.nx + JA_X - 1) / JA_X) * ((g.ny + JA_Y - 1) / JA_Y);
+    const long long slots = (long long) resident * num_sms;
     int best = 1;
     double best_t = 1e300;
-    for (int bz = std::min(g.nz, 32); bz >= 2; --bz) {
-        const double waves = cols * ((g.nz + bz - 1) / bz) / slots;
-        const double t = (bz + 6) * (waves <= 1.0 ? 1.0 : waves + 0.5);
+    for (int bz = std::min(g.nz, 64); bz >= 2; --bz) {
+        const long long blocks = cols * ((g.nz + bz - 1) / bz), rest = blocks % slots;
+        const double last = 0.4 + 0.6 * (double) ((rest + num_sms - 1) / num_sms) / resident;
+        const double t = (bz + 6) * (blocks <= slots ? 1.0 : (double) (blocks / slots) + (rest ? last : 0.0));
         if (t < best_t) {
             best_t = t;
             best = bz;
@@ -279,7 +285,7 @@ cudaError_t launch_jacobian_async(const TI *field, const Geom &g, const JacOut<T
     static std::atomic<unsigned long long> devs{0};
     const cudaError_t attr = opt_in_smem(k_jacobian_async<TI, T, EPI>, smem, devs);
     if (attr != cudaSuccess) return attr;
-    const int bz = jacobian_depth(g, ja_blocks<T>() * num_sms);
+    const int bz = jacobian_depth(g, ja_blocks<T>(), num_sms);
     const long long grid =
         (long long) ((g.nx + JA_X - 1) / JA_X) * ((g.ny + JA_Y - 1) / JA_Y) * ((g.nz + bz - 1) / bz);
     if (grid > INT_MAX) return cudaErrorInvalidConfiguration;
