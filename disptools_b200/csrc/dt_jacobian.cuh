@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
         for (int k = 0; k < 5; ++k) zq[c][k] = TI(0);
     long long off = (z0 - 4) * g.zs + y * g.ys + x;  // of the thread's voxel in plane ze
     int slot = 0;                                    // of plane q
+#pragma unroll(sizeof(T) == 4 ? 5 : 1)
     for (int q = z0 - 2; q <= z1 + 1; ++q, off += g.zs) {
         cp_async_wait_group<JA_D - 1>();
         __syncthreads();
