@@ -1455,19 +1455,14 @@ int jacobian_device_impl(const Geom &g, const T *field, T *J, cudaStream_t s) {
 }
 
 // Whether the adjoint streams its weights by TMA (k_gather_tma) or reads them
-// by plain loads (k_adjoint_gather), by the voxel counts where the two cross:
-// rows a multiple of 16 bytes long, FP32 100^3 64.5 us by TMA and 62.6 plain,
-// 128^3 85 and 110, 160^3 152 and 182; FP64 see above.  Odd widths (weights
-// padded for TMA, their stores and the gradient's unpaired) FP32 129 x 127 x
-// 125 97 and 93, 160 x 161 x 159 170 and 166, 181 x 217 x 181 252 and 262;
-// FP64 334 and 254, 474 and 400, 255 x 255 x 257 1229 and 995.
-template <typename T>
-bool adjoint_streams_weights(const Geom &g) {
-    if (g.order != 4) return false;
-    const long long n = (long long) g.nx * g.ny * g.nz;
-    if ((g.ys * (long long) sizeof(T)) % 16 == 0) return n >= (sizeof(T) == 4 ? 1ll << 20 : FP64_ELEMENTWISE_VOXELS);
-    return sizeof(T) == 4 && n >= 6000000;
-}
+// by plain loads (k_adjoint_gather): a TMA tile is 32 voxels wide, and rows of
+// a third of that and fewer leave too many of its threads idle.  Adjoint by TMA
+// and plain, us: FP32 32^3 17 and 19, 64^3 19 and 26, 101 x 97 x 99 46 and 56,
+// 160^3 97 and 159, 181 x 217 x 181 189 and 247; FP64 32^3 17 and 21, 101 x 97
+// x 99 73 and 77, 160^3 194 and 243, 181 x 217 x 181 335 and 372; 200 x 200 x
+// 17 FP32 46 and 56, FP64 65 and 71; 200 x 200 x 11 46 and 48, 64 and 60;
+// 200 x 200 x 8 38 and 38, 65 and 54.
+bool adjoint_streams_weights(const Geom &g) { return g.order == 4 && g.nx >= 12; }
 
 // The adjoint's path: the weight pass and gather by default, the fused TMA
 // kernel (order 4, a 16-byte-aligned field whose rows are a multiple of 16
@@ -1497,7 +1492,7 @@ int adjoint_device_impl(const Geom &g, const T *field, const T *gJ, T *gout, cud
     // stream waits for the previous call's gather (any stream) before it
     // overwrites W.  Growing the buffer frees the old one, which waits for the
     // device.
-    const bool streams = adjoint_streams_weights<T>(g);
+    const bool streams = adjoint_streams_weights(g);
     Geom gw = g;
     if (streams) {
         const long long v = 16 / (long long) sizeof(T);

@@ -177,15 +177,25 @@ struct PairOf<double> {
     using type = double2;
 };
 template <typename T>
+__device__ __forceinline__ typename PairOf<T>::type pair_of(T a, T b) {
+    typename PairOf<T>::type v;
+    v.x = a;
+    v.y = b;
+    return v;
+}
+__device__ __forceinline__ double2 p_add(double2 a, double2 b) { return pair_of<double>(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 p_mul(double2 a, double2 b) { return pair_of<double>(a.x * b.x, a.y * b.y); }
+// a + w k, each half as the scalar kernels form it: fused in FP32, rounded
+// twice in FP64.
+__device__ __forceinline__ float2 p_tap(float2 w, float2 k, float2 a) { return p_fma(w, k, a); }
+__device__ __forceinline__ double2 p_tap(double2 w, double2 k, double2 a) { return p_add(a, p_mul(w, k)); }
+template <typename T>
 __device__ __forceinline__ typename PairOf<T>::type ld_pair(const T *p) {
     return *reinterpret_cast<const typename PairOf<T>::type *>(p);
 }
 template <typename T>
 __device__ __forceinline__ void st_pair(T *p, T a, T b) {
-    typename PairOf<T>::type v;
-    v.x = a;
-    v.y = b;
-    *reinterpret_cast<typename PairOf<T>::type *>(p) = v;
+    *reinterpret_cast<typename PairOf<T>::type *>(p) = pair_of<T>(a, b);
 }
 
 // 16 bytes of consecutive elements.
@@ -2284,13 +2294,18 @@ cudaError_t launch_jacobian_tma(const CUtensorMap &tm_u, const Geom &g, T *jout,
 // in its own iteration, so a block barrier every B planes is all that
 // guards reuse (loads run LA = S - B iterations ahead).  Warps whose pairs
 // all have their taps at fourth-order voxels (four or more voxels from
-// every face) take constant coefficients; warps near an x face take
-// per-lane coefficients for the x taps (both as FP32 pairs); the others
-// choose each tap's coefficient by the tap voxel's scheme.
+// every face) take constant coefficients.  The others take each tap's
+// coefficient from a table of the tile's columns, rows and planes, in the
+// order of k_adjoint_gather: a tap's scheme along its axis depends on the tap
+// voxel's place on that axis and on whether the voxel is on the two outer
+// layers of another.  Chosen per tap instead, by case, those warps held up
+// their blocks at every plane (SMs busy 73 % of the launch).
 // ------------------------------------------------------------------------
 // GJ: the stages hold C (the weights without their factor gJ) and two boxes
 // of gJ (TXW + 8 columns, TT_Y + 4 rows) at planes ze and q, and each weight
 // is formed as gJ * C where it is read.
+constexpr int GATHER_MAX_BZ = 32;  // planes of a tile at most (wave_depth)
+
 template <typename T, int TXW, bool GJ = false>
 struct GatherTmaLayout {
     static constexpr int XPX = TXW + 2 * TMA_HX;  // W[.][x] box: TXW + 8 columns, TT_Y rows
@@ -2328,6 +2343,10 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, sizeof(T) == 4 ? 3 : 1)
     unsigned char *smem = align_smem_128(smem_dyn);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::BAR_OFF);
     __shared__ int s_fault;
+    // Coefficient of tap t - 2 for each column, row and plane of the tile;
+    // [1]: where another of the voxel's coordinates is on the two outer layers.
+    constexpr int COORDS = TXW + TT_Y + GATHER_MAX_BZ;
+    __shared__ __align__(16) T s_kappa[2][5][COORDS];
 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TPX + tx;
     if (tid == 0) {
@@ -2341,8 +2360,6 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, sizeof(T) == 4 ? 3 : 1)
     }
     __syncthreads();
     const int n[3] = {g.nx, g.ny, g.nz};
-    // Fourth-order coefficients kappa(S_C4, t) by tap, t = -2, -1, 1, 2.
-    const T kc[4] = {FD<T>::one_twelfth, -FD<T>::two_thirds, FD<T>::two_thirds, -FD<T>::one_twelfth};
     uint32_t kbase = 0;  // iterations consumed by this block (mbarrier phases)
 
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -2372,6 +2389,16 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, sizeof(T) == 4 ? 3 : 1)
         };
         if (tid == 0)
             for (int j = 0; j < min(LA, n_it); ++j) issue(j);
+        // Read after the first plane's block barrier.
+        for (int i = tid; i < 10 * COORDS; i += TPX * TYT) {
+            const int other = i / (5 * COORDS), j = i % (5 * COORDS), t = j / COORDS - 2, w = j % COORDS;
+            const int a = w < TXW ? 0 : (w < TXW + TT_Y ? 1 : 2);
+            const int p = (a == 0 ? x0 + w : (a == 1 ? y0 + w - TXW : z0 + w - TXW - TT_Y)) - t;
+            const int kk = p == 0 ? S_FWD
+                         : p == n[a] - 1 ? S_BWD
+                         : (other || p == 1 || p == n[a] - 2) ? S_C2 : S_C4;
+            s_kappa[other][t + 2][w] = p < 0 || p >= n[a] ? T(0) : kappa<T>(kk, t);
+        }
 
         const int x = x0 + 2 * tx;  // this thread's columns: x, x + 1
         const bool pair_in = x + 1 < g.nx;
@@ -2412,9 +2439,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, sizeof(T) == 4 ? 3 : 1)
             // A weight pair gJ * C (GJ) or W as stored.
             auto wmul = [&](P2 w, const T *gp) -> P2 {
                 if constexpr (GJ) {
-                    const P2 gv = ld_pair(gp);
-                    if constexpr (sizeof(T) == 4) return p_mul(w, gv);
-                    else return P2{w.x * gv.x, w.y * gv.y};
+                    return p_mul(w, ld_pair(gp));
                 } else {
                     return w;
                 }
@@ -2445,199 +2470,132 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, sizeof(T) == 4 ? 3 : 1)
                 const int ly = ty + r * TYT, y = y0 + ly;
                 const bool valid = x < g.nx && y < g.ny;
                 T acc[2][3];
-                // Three paths, chosen per warp (a warp is two rows of the
-                // tile, so a voxel's path depends on where it lies, not on the
+                // Two paths, chosen per warp (a warp is two rows of the tile,
+                // so a voxel's path depends on where it lies, not on the
                 // launch): every pair of the warp with all its taps at
                 // fourth-order voxels (four or more voxels from every face);
-                // y and z that deep but x near a face (only the x taps choose
-                // a scheme); the rest.  In FP32 the first two run on pairs.
-                const bool yz_deep = y >= 4 && y <= g.ny - 5 && ze >= 4 && ze <= g.nz - 5;
-                const bool deep = yz_deep && x >= 4 && x + 1 <= g.nx - 5;
-                const bool w_deep = __all_sync(0xffffffffu, deep || !valid);
-                const bool w_yz = __all_sync(0xffffffffu, yz_deep || !valid);
-                auto acc_op = [](T a, T w, T kp) -> T {
-                    if constexpr (sizeof(T) == 4) return __fmaf_rn(w, kp, a);
-                    else return a + w * kp;
-                };
-                bool done = false;
-                if constexpr (sizeof(T) == 4) {
-                    if (w_deep) {
-                        // sum over the axes of (W(+2) - W(-2)) / 12 + (W(-1) - W(+1)) 2/3,
-                        // W(+t) the weight t voxels up the axis: the fourth-order
-                        // taps with the differences formed first, per axis
-                        // independent, for instruction-level parallelism.
-                        const float2 k12 = p_splat(FD<float>::one_twelfth), k23 = p_splat(FD<float>::two_thirds);
+                // the rest.
+                const bool deep = x >= 4 && x + 1 <= g.nx - 5 && y >= 4 && y <= g.ny - 5 && ze >= 4 && ze <= g.nz - 5;
+                const T *gp = gje + (ly + TMA_HY) * XPX + 2 * tx + TMA_HX;  // gJ at (x, y, ze)
+                const T *px = wx + ly * XPX + 2 * tx + TMA_HX;
+                const T *py = wy + (ly + TMA_HY) * TXW + 2 * tx;
+                if (__all_sync(0xffffffffu, deep || !valid)) {
+                    // FP32: the sum over the axes of (W(+2) - W(-2)) / 12 +
+                    // (W(-1) - W(+1)) 2/3, W(+t) the weight t voxels up the
+                    // axis: the fourth-order taps with the differences formed
+                    // first, per axis independent, for instruction-level
+                    // parallelism.  FP64: the taps in order.
+                    const P2 k12 = pair_of<T>(FD<T>::one_twelfth, FD<T>::one_twelfth),
+                             k23 = pair_of<T>(FD<T>::two_thirds, FD<T>::two_thirds);
 #pragma unroll
-                        const T *gp = gje + (ly + TMA_HY) * XPX + 2 * tx + TMA_HX;  // gJ at (x, y, ze)
-                        for (int c = 0; c < 3; ++c) {
-                            const T *px = wx + (c * TT_Y + ly) * XPX + 2 * tx + TMA_HX;
-                            const float2 xm = wmul(ld_pair(px - 2), gp - 2), xc = wmul(ld_pair(px), gp),
-                                         xp = wmul(ld_pair(px + 2), gp + 2);
-                            const T *py = wy + (c * YPY + ly + TMA_HY) * TXW + 2 * tx;
-                            const float2 ym2 = wmul(ld_pair(py - 2 * TXW), gp - 2 * XPX),
-                                         ym1 = wmul(ld_pair(py - TXW), gp - XPX);
-                            const float2 yp1 = wmul(ld_pair(py + TXW), gp + XPX),
-                                         yp2 = wmul(ld_pair(py + 2 * TXW), gp + 2 * XPX);
-                            const float2 d1x = make_float2(__fsub_rn(xm.y, xc.y), __fsub_rn(xc.x, xp.x));
-                            const float2 sx = p_fma(d1x, k23, p_mul(p_sub(xp, xm), k12));
-                            const float2 sy = p_fma(p_sub(ym1, yp1), k23, p_mul(p_sub(yp2, ym2), k12));
-                            const float2 sz = p_fma(p_sub(wq[r][c][1], wq[r][c][3]), k23,
-                                                    p_mul(p_sub(wq[r][c][4], wq[r][c][0]), k12));
-                            const float2 a2 = p_add(p_add(sx, sy), sz);
-                            acc[0][c] = a2.x;
-                            acc[1][c] = a2.y;
-                        }
-                        done = true;
-                    } else if (w_yz) {
-                        // x near a face: per-lane coefficients of the x taps
-                        // (the tap voxel's scheme along x) and of the y and z
-                        // taps (second order when the voxel's x is on the two
-                        // outer layers), in the general path's tap order.
-                        float2 kx[5], kyz[4];
-#pragma unroll
-                        for (int i = 0; i < 5; ++i) {
-                            const int t = i - 2;
-                            float kv[2];
-#pragma unroll
-                            for (int v = 0; v < 2; ++v) {
-                                const int pa = x + v - t;
-                                const int kk = pa == 0 ? S_FWD
-                                             : pa == g.nx - 1 ? S_BWD
-                                             : (pa == 1 || pa == g.nx - 2) ? S_C2 : S_C4;
-                                kv[v] = pa < 0 || pa >= g.nx ? 0.f : kappa<float>(kk, t);
-                            }
-                            kx[i] = make_float2(kv[0], kv[1]);
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int t = i < 2 ? i - 2 : i - 1;
-                            float kv[2];
-#pragma unroll
-                            for (int v = 0; v < 2; ++v) {
-                                const bool x_c2 = x + v <= 1 || x + v >= g.nx - 2;
-                                kv[v] = x_c2 ? kappa<float>(S_C2, t) : kc[i];
-                            }
-                            kyz[i] = make_float2(kv[0], kv[1]);
-                        }
-                        const T *gp = gje + (ly + TMA_HY) * XPX + 2 * tx + TMA_HX;  // gJ at (x, y, ze)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const T *px = wx + (c * TT_Y + ly) * XPX + 2 * tx + TMA_HX;
-                            const float2 xm = wmul(ld_pair(px - 2), gp - 2), xc = wmul(ld_pair(px), gp),
-                                         xp = wmul(ld_pair(px + 2), gp + 2);
-                            const T *py = wy + (c * YPY + ly + TMA_HY) * TXW + 2 * tx;
-                            float2 a2 = p_mul(xp, kx[0]);
-                            a2 = p_fma(make_float2(xc.y, xp.x), kx[1], a2);
-                            a2 = p_fma(xc, kx[2], a2);
-                            a2 = p_fma(make_float2(xm.y, xc.x), kx[3], a2);
-                            a2 = p_fma(xm, kx[4], a2);
-                            a2 = p_fma(wmul(ld_pair(py + 2 * TXW), gp + 2 * XPX), kyz[0], a2);
-                            a2 = p_fma(wmul(ld_pair(py + TXW), gp + XPX), kyz[1], a2);
-                            a2 = p_fma(wmul(ld_pair(py - TXW), gp - XPX), kyz[2], a2);
-                            a2 = p_fma(wmul(ld_pair(py - 2 * TXW), gp - 2 * XPX), kyz[3], a2);
-                            a2 = p_fma(wq[r][c][4], kyz[0], a2);
-                            a2 = p_fma(wq[r][c][3], kyz[1], a2);
-                            a2 = p_fma(wq[r][c][1], kyz[2], a2);
-                            a2 = p_fma(wq[r][c][0], kyz[3], a2);
-                            acc[0][c] = a2.x;
-                            acc[1][c] = a2.y;
-                        }
-                        done = true;
-                    }
-                }
-                if (!done) {
-#pragma unroll
-                    for (int v = 0; v < 2; ++v) {
-                        T a3[3] = {T(0), T(0), T(0)};
-                        if (w_yz) {
-                            // Only x can be outer or penultimate: the x taps
-                            // choose their schemes; the y and z taps are
-                            // fourth order, or second order when the voxel's
-                            // x is on the two outer layers (its tap voxels
-                            // share that x).  Same order as below.
-                            const int xv = x + v;
-                            const bool x_c2 = xv <= 1 || xv >= g.nx - 2;
-#pragma unroll
-                            for (int t = -2; t <= 2; ++t) {
-                                const int pa = xv - t;
-                                if (pa < 0 || pa >= g.nx) continue;
-                                const int kk = pa == 0 ? S_FWD
-                                             : pa == g.nx - 1 ? S_BWD
-                                             : (pa == 1 || pa == g.nx - 2) ? S_C2 : S_C4;
-                                const T kp = kappa<T>(kk, t);
-                                if (kp == T(0)) continue;
-#pragma unroll
-                                for (int c = 0; c < 3; ++c)
-                                    a3[c] = acc_op(a3[c],
-                                                   wmul1(wx[(c * TT_Y + ly) * XPX + 2 * tx + v - t + TMA_HX],
-                                                         gje + (ly + TMA_HY) * XPX + 2 * tx + v - t + TMA_HX),
-                                                   kp);
-                            }
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int t = i < 2 ? i - 2 : i - 1;
-                                if (x_c2 && (t == -2 || t == 2)) continue;
-                                const T kp = x_c2 ? kappa<T>(S_C2, t) : kc[i];
-#pragma unroll
-                                for (int c = 0; c < 3; ++c)
-                                    a3[c] = acc_op(a3[c],
-                                                   wmul1(wy[(c * YPY + ly + TMA_HY - t) * TXW + 2 * tx + v],
-                                                         gje + (ly + TMA_HY - t) * XPX + 2 * tx + v + TMA_HX),
-                                                   kp);
-                            }
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int t = i < 2 ? i - 2 : i - 1;
-                                if (x_c2 && (t == -2 || t == 2)) continue;
-                                const T kp = x_c2 ? kappa<T>(S_C2, t) : kc[i];
-#pragma unroll
-                                for (int c = 0; c < 3; ++c)
-                                    a3[c] = acc_op(a3[c], v ? wq[r][c][2 - t].y : wq[r][c][2 - t].x, kp);
-                            }
+                    for (int c = 0; c < 3; ++c, px += TT_Y * XPX, py += YPY * TXW) {
+                        const P2 xm = wmul(ld_pair(px - 2), gp - 2), xc = wmul(ld_pair(px), gp),
+                                 xp = wmul(ld_pair(px + 2), gp + 2);
+                        const P2 ym2 = wmul(ld_pair(py - 2 * TXW), gp - 2 * XPX), ym1 = wmul(ld_pair(py - TXW), gp - XPX);
+                        const P2 yp1 = wmul(ld_pair(py + TXW), gp + XPX), yp2 = wmul(ld_pair(py + 2 * TXW), gp + 2 * XPX);
+                        P2 a2;
+                        if constexpr (sizeof(T) == 4) {
+                            const P2 d1x = make_float2(__fsub_rn(xm.y, xc.y), __fsub_rn(xc.x, xp.x));
+                            const P2 sx = p_fma(d1x, k23, p_mul(p_sub(xp, xm), k12));
+                            const P2 sy = p_fma(p_sub(ym1, yp1), k23, p_mul(p_sub(yp2, ym2), k12));
+                            const P2 sz = p_fma(p_sub(wq[r][c][1], wq[r][c][3]), k23,
+                                                p_mul(p_sub(wq[r][c][4], wq[r][c][0]), k12));
+                            a2 = p_add(p_add(sx, sy), sz);
                         } else {
-                            // Per tap: the tap voxel p = q - t e_a differs
-                            // from q only along a, so the outer / penultimate
-                            // flags of the other axes come from q
-                            // (src/jacobian.c:70-242).
-                            const int q3[3] = {x + v, y, ze};
-                            bool ob[3], pb[3];
+                            const P2 n12 = pair_of<T>(-k12.x, -k12.x), n23 = pair_of<T>(-k23.x, -k23.x);
+                            a2 = p_mul(xp, k12);
+                            a2 = p_tap(pair_of<T>(xc.y, xp.x), n23, a2);
+                            a2 = p_tap(pair_of<T>(xm.y, xc.x), k23, a2);
+                            a2 = p_tap(xm, n12, a2);
+                            a2 = p_tap(yp2, k12, a2);
+                            a2 = p_tap(yp1, n23, a2);
+                            a2 = p_tap(ym1, k23, a2);
+                            a2 = p_tap(ym2, n12, a2);
+                            a2 = p_tap(wq[r][c][4], k12, a2);
+                            a2 = p_tap(wq[r][c][3], n23, a2);
+                            a2 = p_tap(wq[r][c][1], k23, a2);
+                            a2 = p_tap(wq[r][c][0], n12, a2);
+                        }
+                        acc[0][c] = a2.x;
+                        acc[1][c] = a2.y;
+                    }
+                } else {
+                    const bool xo0 = x <= 1 || x >= g.nx - 2, xo1 = x <= 0 || x >= g.nx - 3;
+                    const bool yo = y <= 1 || y >= g.ny - 2, zo = ze <= 1 || ze >= g.nz - 2;
+                    P2 a2[3];
+                    {
+                        const T *kx = &s_kappa[yo || zo][0][2 * tx];
+                        const P2 k0 = ld_pair(kx), k1 = ld_pair(kx + COORDS), k2 = ld_pair(kx + 2 * COORDS),
+                                 k3 = ld_pair(kx + 3 * COORDS), k4 = ld_pair(kx + 4 * COORDS);
 #pragma unroll
-                            for (int b = 0; b < 3; ++b) {
-                                ob[b] = q3[b] == 0 || q3[b] == n[b] - 1;
-                                pb[b] = q3[b] == 1 || q3[b] == n[b] - 2;
-                            }
+                        for (int c = 0; c < 3; ++c) {
+                            const T *p = px + c * TT_Y * XPX;
+                            const P2 xm = wmul(ld_pair(p - 2), gp - 2), xc = wmul(ld_pair(p), gp),
+                                     xp = wmul(ld_pair(p + 2), gp + 2);
+                            a2[c] = p_mul(xp, k0);
+                            a2[c] = p_tap(pair_of<T>(xc.y, xp.x), k1, a2[c]);
+                            a2[c] = p_tap(xc, k2, a2[c]);
+                            a2[c] = p_tap(pair_of<T>(xm.y, xc.x), k3, a2[c]);
+                            a2[c] = p_tap(xm, k4, a2[c]);
+                        }
+                    }
+                    const T *ky0 = &s_kappa[xo0 || zo][0][TXW + ly], *ky1 = &s_kappa[xo1 || zo][0][TXW + ly];
 #pragma unroll
-                            for (int a = 0; a < 3; ++a) {
-                                const bool o_other = (a != 0 && ob[0]) || (a != 1 && ob[1]) || (a != 2 && ob[2]);
-                                const bool p_other = (a != 0 && pb[0]) || (a != 1 && pb[1]) || (a != 2 && pb[2]);
+                    for (int t = -2; t <= 2; ++t) {
+                        const P2 ky = pair_of<T>(ky0[(t + 2) * COORDS], ky1[(t + 2) * COORDS]);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+                            a2[c] = p_tap(wmul(ld_pair(py + c * YPY * TXW - t * TXW), gp - t * XPX), ky, a2[c]);
+                    }
+                    const int wz0 = TXW + TT_Y + ze - z0;
+                    const T *kz0 = &s_kappa[xo0 || yo][0][wz0], *kz1 = &s_kappa[xo1 || yo][0][wz0];
+#pragma unroll
+                    for (int t = -2; t <= 2; ++t) {
+                        const P2 kz = pair_of<T>(kz0[(t + 2) * COORDS], kz1[(t + 2) * COORDS]);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) a2[c] = p_tap(wq[r][c][2 - t], kz, a2[c]);
+                    }
+                    bool finite = true;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        acc[0][c] = a2[c].x;
+                        acc[1][c] = a2[c].y;
+                        finite = finite && isfinite(a2[c].x) && (!pair_in || isfinite(a2[c].y));
+                    }
+                    // A weight that is not finite counts only where its
+                    // coefficient is not zero: such sums are formed again
+                    // from the taps that have one.
+                    if (valid && !finite) {
+#pragma unroll 1
+                        for (int v = 0; v < 2; ++v) {
+                            T a3[3] = {T(0), T(0), T(0)};
+                            const bool xo = v ? xo1 : xo0;
+                            const int others[3] = {yo || zo, xo || zo, xo || yo};
+                            const int place[3] = {2 * tx + v, TXW + ly, wz0};
+#pragma unroll
+                            for (int a = 0; a < 3; ++a)
 #pragma unroll
                                 for (int t = -2; t <= 2; ++t) {
-                                    const int pa = q3[a] - t;
-                                    if (pa < 0 || pa >= n[a]) continue;
-                                    const bool outer = o_other || pa == 0 || pa == n[a] - 1;
-                                    const bool pen = p_other || pa == 1 || pa == n[a] - 2;
-                                    const int kk = outer ? (pa == 0 ? S_FWD : (pa == n[a] - 1 ? S_BWD : S_C2))
-                                                         : (pen ? S_C2 : S_C4);
-                                    const T kp = kappa<T>(kk, t);
+                                    const T kp = s_kappa[others[a]][t + 2][place[a]];
                                     if (kp == T(0)) continue;
 #pragma unroll
                                     for (int c = 0; c < 3; ++c) {
                                         T w;
                                         if (a == 0)
-                                            w = wmul1(wx[(c * TT_Y + ly) * XPX + 2 * tx + v - t + TMA_HX],
-                                                      gje + (ly + TMA_HY) * XPX + 2 * tx + v - t + TMA_HX);
+                                            w = wmul1(px[c * TT_Y * XPX + v - t], gp + v - t);
                                         else if (a == 1)
-                                            w = wmul1(wy[(c * YPY + ly + TMA_HY - t) * TXW + 2 * tx + v],
-                                                      gje + (ly + TMA_HY - t) * XPX + 2 * tx + v + TMA_HX);
+                                            w = wmul1(py[(c * YPY - t) * TXW + v], gp + v - t * XPX);
                                         else
                                             w = v ? wq[r][c][2 - t].y : wq[r][c][2 - t].x;
-                                        a3[c] = acc_op(a3[c], w, kp);
+                                        if constexpr (sizeof(T) == 4) a3[c] = __fmaf_rn(w, kp, a3[c]);
+                                        else a3[c] = a3[c] + w * kp;
                                     }
                                 }
-                            }
-                        }
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) acc[v][c] = a3[c];
+                            for (int c = 0; c < 3; ++c)
+                                if (v) acc[1][c] = a3[c];
+                                else acc[0][c] = a3[c];
+                        }
                     }
                 }
                 if (!valid) continue;
@@ -2709,7 +2667,7 @@ cudaError_t launch_gather_tma_v(const CUtensorMap &tm_wx, const CUtensorMap &tm_
     const int tiles_x = (g.nx + TXW - 1) / TXW, tiles_y = (g.ny + TT_Y - 1) / TT_Y;
     const int cols = tiles_x * tiles_y;
     const int slots = std::max(1, gather_blocks_v<T, TXW, TYT, GJ>()) * num_sms;  // resident blocks
-    const int bz = wave_depth(cols, g.nz, slots);
+    const int bz = std::min(wave_depth(cols, g.nz, slots), GATHER_MAX_BZ);
     const int ntiles = cols * ((g.nz + bz - 1) / bz);
     const int grid = std::min(ntiles, slots);
     k_gather_tma<T, TXW, TYT, GJ><<<grid, dim3(TXW / 2, TYT), smem, s>>>(tm_wx, tm_wy, tm_wz, tm_gj, g, gout, tiles_x,

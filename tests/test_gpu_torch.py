@@ -266,3 +266,41 @@ def test_adjoint_of_odd_widths(oracle, oracle_pd2, shape, order):
         g = torch_ops.jacobian_adjoint_raw(torch.from_numpy(u).to(dtype).cuda(), torch.from_numpy(w).to(dtype).cuda(),
                                            sp, order).double().cpu().numpy()
         assert abs(np.sum(g * v) - np.sum(w * dJ)) <= tol * scale
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 12), (4, 6, 13), (3, 40, 16), (70, 3, 33), (8, 9, 11), (9, 7, 64)])
+def test_adjoint_taps_near_faces(oracle, oracle_pd2, shape):
+    """Volumes in which most taps choose a scheme, on both sides of the widths
+    that stream their weights."""
+    test_adjoint_of_odd_widths(oracle, oracle_pd2, shape, 4)
+
+
+@pytest.mark.parametrize("shape", [(12, 20, 48), (12, 20, 45)])
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_adjoint_keeps_infinities_local(shape, value):
+    """A weight that is not finite reaches the voxels that have a tap on it
+    (those that a large finite one changes) and no others, with or without
+    the saved cofactors."""
+    import torch
+    from disptools_b200 import torch_ops
+    rng = np.random.default_rng(3)
+    u = rng.normal(scale=0.2, size=(3,) + shape)
+    w = rng.standard_normal(shape)
+
+    def through_autograd(field, weight):
+        leaf = field.clone().requires_grad_(True)
+        return torch.autograd.grad(torch_ops.jacobian(leaf), leaf, weight)[0]
+
+    for dtype in (torch.float32, torch.float64):
+        field, weight = torch.from_numpy(u).to(dtype).cuda(), torch.from_numpy(w).to(dtype).cuda()
+        for adjoint in (torch_ops.jacobian_adjoint_raw, through_autograd):
+            for place in ((0, 0, 0), (1, 10, 31), (6, 1, 32), (6, 10, 1), (6, 10, 20), (11, 19, shape[2] - 2)):
+                results = []
+                for v in (0.0, 1e30, value):
+                    weight[place] = v
+                    results.append(adjoint(field, weight))
+                zero, large, bad = results
+                reached = large != zero
+                assert torch.equal(~torch.isfinite(bad), reached)
+                assert torch.equal(bad[~reached], zero[~reached])
+                weight[place] = float(w[place])
