@@ -29,12 +29,19 @@
 
 namespace dtb {
 
-constexpr int JA_X = BX, JA_Y = BY, JA_NT = JA_X * JA_Y;
-constexpr int JA_PX = JA_X + 4, JA_PY = JA_Y + 4, JA_ROWS = 3 * JA_PY, JA_PLANE = JA_ROWS * JA_PX;
-constexpr int JA_D = 3, JA_NS = JA_D + 3;
-// Copies: 216 threads take the 36 columns of 6 rows at a time, two sweeps a component.
-constexpr int JA_RG = JA_PY / 2;
-static_assert(JA_RG * JA_PX <= JA_NT);
+constexpr int JA_NT = 256, JA_D = 3, JA_NS = JA_D + 3;
+
+// Tiles are TX voxels wide and JA_NT / TX high: 32 x 8, and 8 x 32 for volumes
+// at most 16 voxels wide, which would leave most of a 32-wide tile idle.
+template <int TX>
+struct JaTile {
+    static constexpr int X = TX, Y = JA_NT / TX;
+    static constexpr int PX = X + 4, PY = Y + 4, CELLS = PX * PY, PLANE = 3 * CELLS;
+    // Copies: the threads take the columns of half a component's rows at a time.
+    static constexpr int RG = PY / 2;
+    static_assert(RG * PX <= JA_NT && PY % 2 == 0);
+};
+constexpr int JA_NARROW = 16;
 
 // Resident blocks per SM: 32 warps at 64 registers (FP32), 16 at 128 (FP64).
 template <typename T>
@@ -94,15 +101,15 @@ struct CentralWeights {
 // and has code without a choice per voxel.  Other voxels take fourth-order
 // differences where `c4`, and are second order along every axis elsewhere
 // (schemes_at), one-sided where they lie on a face.
-template <typename TI, typename T>
+template <int PX, int CELLS, typename TI, typename T>
 __device__ __forceinline__ void stencil_voxel(const TI *p, const TI (&zq)[3][5], int x, int y, int z, const Geom &g,
                                               const T (&ih)[3], bool deep, bool c4, T (&a)[3][3]) {
     auto central = [&](const CentralWeights<T> &w, auto second) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const TI *q = p + c * JA_PY * JA_PX;
+            const TI *q = p + c * CELLS;
             a[c][0] = w((T) q[1] - (T) q[-1], second((T) q[2] - (T) q[-2]), 0);
-            a[c][1] = w((T) q[JA_PX] - (T) q[-JA_PX], second((T) q[2 * JA_PX] - (T) q[-2 * JA_PX]), 1);
+            a[c][1] = w((T) q[PX] - (T) q[-PX], second((T) q[2 * PX] - (T) q[-2 * PX]), 1);
             a[c][2] = w((T) zq[c][3] - (T) zq[c][1], second((T) zq[c][4] - (T) zq[c][0]), 2);
         }
     };
@@ -114,29 +121,29 @@ __device__ __forceinline__ void stencil_voxel(const TI *p, const TI (&zq)[3][5],
     if (x == 0) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const TI *q = p + c * JA_PY * JA_PX;
+            const TI *q = p + c * CELLS;
             a[c][0] = fd_fwd<T>(q[0], q[1], q[2], ih[0]);
         }
     }
     if (x == g.nx - 1) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const TI *q = p + c * JA_PY * JA_PX;
+            const TI *q = p + c * CELLS;
             a[c][0] = fd_bwd<T>(q[0], q[-1], q[-2], ih[0]);
         }
     }
     if (y == 0) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const TI *q = p + c * JA_PY * JA_PX;
-            a[c][1] = fd_fwd<T>(q[0], q[JA_PX], q[2 * JA_PX], ih[1]);
+            const TI *q = p + c * CELLS;
+            a[c][1] = fd_fwd<T>(q[0], q[PX], q[2 * PX], ih[1]);
         }
     }
     if (y == g.ny - 1) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const TI *q = p + c * JA_PY * JA_PX;
-            a[c][1] = fd_bwd<T>(q[0], q[-JA_PX], q[-2 * JA_PX], ih[1]);
+            const TI *q = p + c * CELLS;
+            a[c][1] = fd_bwd<T>(q[0], q[-PX], q[-2 * PX], ih[1]);
         }
     }
     if (z == 0) {
@@ -149,41 +156,42 @@ __device__ __forceinline__ void stencil_voxel(const TI *p, const TI (&zq)[3][5],
     }
 }
 
-template <typename TI, typename T, int EPI>
+template <typename TI, typename T, int EPI, int TX>
 __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
     k_jacobian_async(const TI *__restrict__ field, const Geom g, const JacOut<T> out, int bz) {
+    using L = JaTile<TX>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TI *ring = reinterpret_cast<TI *>(smem_raw);
-    const int tid = threadIdx.x, tx = tid % JA_X, ty = tid / JA_X;
-    const int tiles_x = (g.nx + JA_X - 1) / JA_X, tiles_y = (g.ny + JA_Y - 1) / JA_Y;
+    const int tid = threadIdx.x, tx = tid % L::X, ty = tid / L::X;
+    const int tiles_x = (g.nx + L::X - 1) / L::X, tiles_y = (g.ny + L::Y - 1) / L::Y;
     const int txy = (int) blockIdx.x / tiles_x;
-    const int x0 = ((int) blockIdx.x - txy * tiles_x) * JA_X, y0 = (txy % tiles_y) * JA_Y, z0 = (txy / tiles_y) * bz;
+    const int x0 = ((int) blockIdx.x - txy * tiles_x) * L::X, y0 = (txy % tiles_y) * L::Y, z0 = (txy / tiles_y) * bz;
     const int z1 = min(z0 + bz, g.nz);
     // Box positions outside the volume stay zero: their x and y are the same
     // in every plane, planes below it are never copied, planes above it are
     // cleared.
-    if (z0 < 2 || y0 < 2 || x0 < 2 || y0 + JA_Y + 2 > g.ny || x0 + JA_X + 2 > g.nx) {
-        for (int i = tid; i < JA_NS * JA_PLANE; i += JA_NT) ring[i] = TI(0);
+    if (z0 < 2 || y0 < 2 || x0 < 2 || y0 + L::Y + 2 > g.ny || x0 + L::X + 2 > g.nx) {
+        for (int i = tid; i < JA_NS * L::PLANE; i += JA_NT) ring[i] = TI(0);
         __syncthreads();
     }
-    const int rg = tid / JA_PX, col = tid - rg * JA_PX;
+    const int rg = tid / L::PX, col = tid - rg * L::PX;
     const int gx = x0 - 2 + col, gy = y0 - 2 + rg;
-    const bool col_ok = rg < JA_RG && gx >= 0 && gx < g.nx;
-    const bool lo = col_ok && gy >= 0 && gy < g.ny, hi = col_ok && gy + JA_RG >= 0 && gy + JA_RG < g.ny;
+    const bool col_ok = rg < L::RG && gx >= 0 && gx < g.nx;
+    const bool lo = col_ok && gy >= 0 && gy < g.ny, hi = col_ok && gy + L::RG >= 0 && gy + L::RG < g.ny;
     const TI *src = field + ((z0 - 2) * g.zs + gy * g.ys + gx);  // in the next plane to copy
     // Copies plane zp (tile and halo) into its slot; always one group.
     auto load_plane = [&](int zp, int slot) {
         if (zp >= 0 && zp <= z1 + 1) {
-            TI *dst = ring + slot * JA_PLANE + tid;
+            TI *dst = ring + slot * L::PLANE + tid;
             if (zp < g.nz) {
-                const TI *up = src + JA_RG * g.ys;
+                const TI *up = src + L::RG * g.ys;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    if (lo) cp_async_elem<(int) sizeof(TI)>(dst + c * JA_PY * JA_PX, src + c * g.cs);
-                    if (hi) cp_async_elem<(int) sizeof(TI)>(dst + (c * JA_PY + JA_RG) * JA_PX, up + c * g.cs);
+                    if (lo) cp_async_elem<(int) sizeof(TI)>(dst + c * L::CELLS, src + c * g.cs);
+                    if (hi) cp_async_elem<(int) sizeof(TI)>(dst + c * L::CELLS + L::RG * L::PX, up + c * g.cs);
                 }
             } else {
-                for (int i = tid; i < JA_PLANE; i += JA_NT) ring[slot * JA_PLANE + i] = TI(0);
+                for (int i = tid; i < L::PLANE; i += JA_NT) ring[slot * L::PLANE + i] = TI(0);
             }
         }
         src += g.zs;
@@ -195,9 +203,10 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
     const bool in_xy = x < g.nx && y < g.ny;
     const T ih[3] = {(T) g.ih[0], (T) g.ih[1], (T) g.ih[2]};
     const bool row_in = y >= 2 && y <= g.ny - 3 && g.order == 4;
-    const bool tile_in = row_in && x0 >= 2 && x0 + JA_X - 1 <= g.nx - 3;
+    // A warp of a wide tile is one row of it.
+    const bool tile_in = TX == 32 && row_in && x0 >= 2 && x0 + L::X - 1 <= g.nx - 3;
     const bool voxel_in = row_in && x >= 2 && x <= g.nx - 3;
-    const int own = (ty + 2) * JA_PX + tx + 2;
+    const int own = (ty + 2) * L::PX + tx + 2;
     TI zq[3][5];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
@@ -211,12 +220,12 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
         __syncthreads();
         // The slot of plane q + D held plane q - 3, the last centre plane.
         load_plane(q + JA_D, slot + JA_D < JA_NS ? slot + JA_D : slot + JA_D - JA_NS);
-        const TI *pl = ring + slot * JA_PLANE + own;
+        const TI *pl = ring + slot * L::PLANE + own;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) zq[c][k] = zq[c][k + 1];
-            zq[c][4] = pl[c * JA_PY * JA_PX];
+            zq[c][4] = pl[c * L::CELLS];
         }
         const int ze = q - 2;
         const int se = slot >= 2 ? slot - 2 : slot - 2 + JA_NS;
@@ -228,7 +237,7 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
         if constexpr (EPI == JAC_LOG) pre = out.first ? T(0) : out.acc[off];
         const bool plane_in = ze >= 2 && ze <= g.nz - 3;
         T a[3][3];
-        stencil_voxel<TI, T>(ring + se * JA_PLANE + own, zq, x, y, ze, g, ih, tile_in && plane_in,
+        stencil_voxel<L::PX, L::CELLS, TI, T>(ring + se * L::PLANE + own, zq, x, y, ze, g, ih, tile_in && plane_in,
                              voxel_in && plane_in, a);
         if constexpr (EPI == JAC_MAP) {
             out.J[off] = det_i_plus<T>(a);
@@ -263,8 +272,7 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
 // two more to start; blocks run in waves of `slots`, of which the last is
 // shorter where it leaves the SMs fewer than their `resident` blocks (a block
 // alone on an SM runs faster, though not in proportion).
-inline int jacobian_depth(const Geom &g, int resident, int num_sms) {
-    const long long cols = (long long) ((g.nx + JA_X - 1) / JA_X) * ((g.ny + JA_Y - 1) / JA_Y);
+inline int jacobian_depth(const Geom &g, long long cols, int resident, int num_sms) {
     const long long slots = (long long) resident * num_sms;
     int best = 1;
     double best_t = 1e300;
@@ -280,19 +288,26 @@ inline int jacobian_depth(const Geom &g, int resident, int num_sms) {
     return best;
 }
 
-template <typename TI, typename T, int EPI>
-cudaError_t launch_jacobian_async(const TI *field, const Geom &g, const JacOut<T> &out, int num_sms, cudaStream_t s) {
-    constexpr int smem = JA_NS * JA_PLANE * (int) sizeof(TI);
+template <typename TI, typename T, int EPI, int TX>
+cudaError_t launch_jacobian_tiles(const TI *field, const Geom &g, const JacOut<T> &out, int num_sms, cudaStream_t s) {
+    using L = JaTile<TX>;
+    constexpr int smem = JA_NS * L::PLANE * (int) sizeof(TI);
     static std::atomic<unsigned long long> devs{0};
-    const cudaError_t attr = opt_in_smem(k_jacobian_async<TI, T, EPI>, smem, devs);
+    const cudaError_t attr = opt_in_smem(k_jacobian_async<TI, T, EPI, TX>, smem, devs);
     if (attr != cudaSuccess) return attr;
-    const int bz = jacobian_depth(g, ja_blocks<T>(), num_sms);
-    const long long grid =
-        (long long) ((g.nx + JA_X - 1) / JA_X) * ((g.ny + JA_Y - 1) / JA_Y) * ((g.nz + bz - 1) / bz);
+    const long long cols = (long long) ((g.nx + L::X - 1) / L::X) * ((g.ny + L::Y - 1) / L::Y);
+    const int bz = jacobian_depth(g, cols, ja_blocks<T>(), num_sms);
+    const long long grid = cols * ((g.nz + bz - 1) / bz);
     if (grid > INT_MAX) return cudaErrorInvalidConfiguration;
-    k_jacobian_async<TI, T, EPI><<<(unsigned) grid, JA_NT, smem, s>>>(field, g, out, bz);
+    k_jacobian_async<TI, T, EPI, TX><<<(unsigned) grid, JA_NT, smem, s>>>(field, g, out, bz);
     count_launch();
     return cudaGetLastError();
+}
+
+template <typename TI, typename T, int EPI>
+cudaError_t launch_jacobian_async(const TI *field, const Geom &g, const JacOut<T> &out, int num_sms, cudaStream_t s) {
+    if (g.nx <= JA_NARROW) return launch_jacobian_tiles<TI, T, EPI, 8>(field, g, out, num_sms, s);
+    return launch_jacobian_tiles<TI, T, EPI, 32>(field, g, out, num_sms, s);
 }
 
 template <typename T>

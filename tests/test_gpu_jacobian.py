@@ -142,6 +142,13 @@ def test_any_layout_kernel_at_tile_edges(oracle, oracle_pd2, shape, order):
             assert rel_err(J2.double().cpu().numpy(), ref) <= tol
 
 
+@pytest.mark.parametrize("shape", [(40, 5, 3), (5, 33, 8), (4, 31, 9), (9, 65, 15), (3, 34, 16), (5, 33, 17)])
+@pytest.mark.parametrize("order", [4, 2])
+def test_any_layout_kernel_on_narrow_volumes(oracle, oracle_pd2, shape, order):
+    """The same around its 8 x 32 tiles and the width that takes them."""
+    test_any_layout_kernel_at_tile_edges(oracle, oracle_pd2, shape, order)
+
+
 def test_any_layout_kernel_keeps_infinities_local(oracle):
     """An infinite value reaches only the voxels whose schemes read it, also
     on the second-order outer layers."""
