@@ -33,6 +33,7 @@ UNITS = [
     ("dt_kernels_f32.cu", []),
     ("dt_kernels_f64.cu", ["-fmad=false"]),
     ("dt_capi.cu", []),
+    ("dt_hostcopy.cu", []),
     ("dt_noalloc.cu", []),
     ("dt_resample.cu", []),
     ("dt_io.cpp", []),

@@ -1229,6 +1229,8 @@ int solve_host(int algorithm, int count, const dtb_volume *vols, const dtb_param
     if (rc != DTB_OK) return rc;
     Carve cv{base};
     double *stage = is_double ? nullptr : cv.take<double>(stage_elems);
+    ResultPages pages;
+    for (int i = 0; i < count; ++i) pages.populate(vols[i].field, 3 * vols[i].nx * vols[i].ny * vols[i].nz * sizeof(double));
     std::vector<DevVol<T>> dv(count);
     for (int i = 0; i < count; ++i) {
         const dtb_volume &v = vols[i];
@@ -1237,18 +1239,18 @@ int solve_host(int algorithm, int count, const dtb_volume *vols, const dtb_param
         T *Jt = cv.take<T>(N);
         uint8_t *mask = cv.take<uint8_t>(N);
         if (is_double) {
-            DTB_CUDA(cudaMemcpyAsync(field, v.field, 3 * N * sizeof(double), cudaMemcpyHostToDevice, stream));
-            DTB_CUDA(cudaMemcpyAsync(Jt, v.J, N * sizeof(double), cudaMemcpyHostToDevice, stream));
+            DTB_CUDA(copy_from_host(field, v.field, 3 * N * sizeof(double), stream));
+            DTB_CUDA(copy_from_host(Jt, v.J, N * sizeof(double), stream));
         } else {
             // The stage is reused by every volume: stream order puts each
             // copy after the previous conversion.
-            DTB_CUDA(cudaMemcpyAsync(stage, v.field, 3 * N * sizeof(double), cudaMemcpyHostToDevice, stream));
+            DTB_CUDA(copy_from_host(stage, v.field, 3 * N * sizeof(double), stream));
             DTB_CUDA(launch_convert<T>(stage, 1, field, 3 * (long long) N, stream));
-            DTB_CUDA(cudaMemcpyAsync(stage, v.J, N * sizeof(double), cudaMemcpyHostToDevice, stream));
+            DTB_CUDA(copy_from_host(stage, v.J, N * sizeof(double), stream));
             DTB_CUDA(launch_convert<T>(stage, 1, Jt, (long long) N, stream));
         }
         static_assert(sizeof(bool) == 1, "bool must be one byte");
-        DTB_CUDA(cudaMemcpyAsync(mask, v.mask, N, cudaMemcpyHostToDevice, stream));
+        DTB_CUDA(copy_from_host(mask, v.mask, N, stream));
         dv[i] = DevVol<T>{make_geom(v.nx, v.ny, v.nz, v.dx, v.dy, v.dz), Jt, mask, field};
     }
     rc = solve_device_on<T>(e, algorithm, dv, p, stats, precision);
@@ -1261,10 +1263,10 @@ int solve_host(int algorithm, int count, const dtb_volume *vols, const dtb_param
         const dtb_volume &v = vols[i];
         const size_t N = v.nx * v.ny * v.nz;
         if (is_double) {
-            DTB_CUDA(cudaMemcpyAsync(v.field, dv[i].field, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, stream));
+            DTB_CUDA(copy_to_host(v.field, dv[i].field, 3 * N * sizeof(double), stream));
         } else {
             DTB_CUDA(launch_to_double<T>(dv[i].field, stage, 3 * (long long) N, stream));
-            DTB_CUDA(cudaMemcpyAsync(v.field, stage, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, stream));
+            DTB_CUDA(copy_to_host(v.field, stage, 3 * N * sizeof(double), stream));
         }
     }
     DTB_CUDA(cudaStreamSynchronize(stream));
@@ -1723,6 +1725,7 @@ extern "C" int dtb_release_device_memory(void) {
             (*pool)[dev] = Workspace{};
         }
     }
+    release_host_staging();
     // The cached step graph points into the freed workspace.
     if ((int) g_engines.size() > dev && g_engines[dev]) {
         for (cudaGraphExec_t &x : g_engines[dev]->exec) {
@@ -1744,22 +1747,25 @@ extern "C" void jacobian_dynamic(const size_t nx, const size_t ny, const size_t 
         return;
     }
     const size_t N = nx * ny * nz;
-    double *df = nullptr, *dJ = nullptr;
-    if (cudaMalloc(&df, 3 * N * sizeof(double)) != cudaSuccess || cudaMalloc(&dJ, N * sizeof(double)) != cudaSuccess) {
+    const size_t field_elems = (3 * N + 31) / 32 * 32;
+    double *df = nullptr;
+    if (cudaMalloc(&df, (field_elems + N) * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(df);
         set_error(__LINE__, __func__, "cannot allocate device buffers");
         return;
     }
-    cudaError_t e = cudaMemcpy(df, f, 3 * N * sizeof(double), cudaMemcpyHostToDevice);
+    double *dJ = df + field_elems;
+    ResultPages pages;
+    pages.populate(J, N * sizeof(double));
+    cudaError_t e = copy_from_host(df, f, 3 * N * sizeof(double), nullptr);
     if (e == cudaSuccess && dtb_jacobian_device(DTB_PRECISION_FP64, 4, nx, ny, nz, dx, dy, dz, df, dJ, nullptr) == DTB_OK)
-        e = cudaMemcpy(J, dJ, N * sizeof(double), cudaMemcpyDeviceToHost);
+        e = copy_to_host(J, dJ, N * sizeof(double), nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error(__LINE__, __func__, cudaGetErrorString(e));
     }
     cudaFree(df);
-    cudaFree(dJ);
 }
 
 // src/jacobian.c:29-55, on the device.
@@ -1773,9 +1779,10 @@ extern "C" void regularise(const size_t nx, const size_t ny, const size_t nz, do
         set_error(__LINE__, __func__, "cannot allocate device buffers");
         return;
     }
-    cudaError_t e = cudaMemcpy(dJ, J, N * sizeof(double), cudaMemcpyHostToDevice);
+    cudaError_t e = copy_from_host(dJ, J, N * sizeof(double), nullptr);
     if (e == cudaSuccess) e = launch_regularise<double>(dJ, (long long) N, epsilon, nullptr);
-    if (e == cudaSuccess) e = cudaMemcpy(J, dJ, N * sizeof(double), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = copy_to_host(J, dJ, N * sizeof(double), nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error(__LINE__, __func__, cudaGetErrorString(e));

@@ -686,7 +686,7 @@ struct Slab {
 };
 
 // Pinned copies of the state, two a solve (one per batch of steps in flight).
-// Kept for later solves: as many as have run at the same time.
+// Up to MAX_SPARE are kept for later solves.
 struct HostStates {
     MatchState *p = nullptr;
     HostStates() {
@@ -705,13 +705,20 @@ struct HostStates {
     }
     ~HostStates() {
         if (!p) return;
-        std::lock_guard<std::mutex> lock(mutex());
-        spare().push_back(p);
+        {
+            std::lock_guard<std::mutex> lock(mutex());
+            if (spare().size() < MAX_SPARE) {
+                spare().push_back(p);
+                return;
+            }
+        }
+        cudaFreeHost(p);
     }
     HostStates(const HostStates &) = delete;
     HostStates &operator=(const HostStates &) = delete;
 
 private:
+    static constexpr size_t MAX_SPARE = 8;
     static std::mutex &mutex() {
         static std::mutex m;
         return m;
@@ -827,8 +834,8 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
     M_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
     M_CUDA(cudaMemcpyAsync(st, &host.p[0], sizeof init, cudaMemcpyHostToDevice, s));
     if (!device) {
-        M_CUDA(cudaMemcpyAsync(dfield, field, 3 * n * sizeof(double), cudaMemcpyHostToDevice, s));
-        M_CUDA(cudaMemcpyAsync(const_cast<double *>(dJ), J, n * sizeof(double), cudaMemcpyHostToDevice, s));
+        M_CUDA(copy_from_host(dfield, field, 3 * n * sizeof(double), s));
+        M_CUDA(copy_from_host(const_cast<double *>(dJ), J, n * sizeof(double), s));
     }
     k_match_prepare<<<grid_for(n), 256, 0, s>>>(dfield, dJ, (int) nx, (int) ny, (int) nz, dx, dy, dz, pos[0],
                                                 pos[0] + n, pos[0] + 2 * n, tv);
@@ -900,7 +907,7 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
                                                dfield);
     count_launch();
     M_CUDA(cudaGetLastError());
-    if (!device) M_CUDA(cudaMemcpyAsync(field, dfield, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (!device) M_CUDA(copy_to_host(field, dfield, 3 * n * sizeof(double), s));
     M_CUDA(cudaStreamSynchronize(s));
     if (stats) {
         std::memset(stats, 0, sizeof *stats);

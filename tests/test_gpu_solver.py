@@ -446,3 +446,31 @@ def test_thin_tiles_equal_deep_tiles(monkeypatch, algorithm, shape):
     deep, sd = dt.solve(Jt, mask, algorithm=algorithm, precision="fp64", it_max=12)
     assert dt.tile_config()["bz"] == 32 and st["iterations"] == sd["iterations"]
     np.testing.assert_array_equal(thin, deep)
+
+
+@pytest.mark.parametrize("shape", [(55, 56, 56), (56, 56, 57), (81, 82, 83)])
+def test_host_arrays_through_staging(shape):
+    """Host arrays on both sides of the size that goes through pinned chunks,
+    at an odd place of a fresh array: the device call's result, nothing
+    written outside it, the same from threads at once and after a release."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    import torch
+
+    from disptools_b200 import api, torch_ops
+    rng = np.random.default_rng(1)
+    J = 1.0 + 0.05 * rng.standard_normal(shape)
+    mask = np.ones(shape, bool)
+    n = 3 * int(np.prod(shape))
+    buffer = np.zeros(n + 1031)
+    field = buffer[517:517 + n].reshape((3,) + shape)
+    api.solve_batched([(J, mask, field)], precision="fp64", inplace=True, it_max=4)
+    want = torch.zeros((3,) + shape, dtype=torch.float64, device="cuda")
+    torch_ops.solve(torch.from_numpy(J).cuda(), torch.from_numpy(mask).cuda(), want, it_max=4)
+    np.testing.assert_array_equal(field, want.cpu().numpy())
+    assert not buffer[:517].any() and not buffer[517 + n:].any()
+    dt.release_device_memory()
+    map_want = torch_ops.jacobian_raw(want).cpu().numpy()
+    with ThreadPoolExecutor(3) as pool:
+        for got in pool.map(api.jacobian, [field] * 6):
+            np.testing.assert_array_equal(got, map_want)
