@@ -1044,6 +1044,9 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
         int s0 = (int) (kbase % L::S), s1 = 0, s2 = 0;
         uint32_t phase_bit = (kbase / L::S) & 1u;
         int ps = 0, ps1 = 0;
+        // Unrolled over the three planes of P_z terms, which then stay where
+        // they are (FP32; 24 volumes of 192^3 at most: 327 -> 314 us a launch).
+#pragma unroll(sizeof(T) == 4 ? 3 : 1)
         for (int it = 0; it < n_it; ++it, zoff += g.zs) {
             const bool ok = mbar_wait_bounded(&bars[s0], phase_bit);
             const int q = z0 - 2 + it;
