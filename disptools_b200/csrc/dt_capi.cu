@@ -1494,17 +1494,18 @@ int adjoint_device_impl(const Geom &g, const T *field, const T *gJ, T *gout, cud
     // stream waits for the previous call's gather (any stream) before it
     // overwrites W.  Growing the buffer frees the old one, which waits for the
     // device.
-    const bool streams = adjoint_streams_weights(g);
+    auto scratch = [](const Geom &w) { return 9 * (size_t) ((w.cs + 63) / 64 * 64) * sizeof(T) + 256; };
     Geom gw = g;
-    if (streams) {
-        const long long v = 16 / (long long) sizeof(T);
-        gw.ys = (g.nx + v - 1) / v * v;
-        gw.zs = gw.ys * g.ny;
-        gw.cs = gw.zs * g.nz;
-    }
+    const long long v = 16 / (long long) sizeof(T);
+    gw.ys = (g.nx + v - 1) / v * v;
+    gw.zs = gw.ys * g.ny;
+    gw.cs = gw.zs * g.nz;
+    // Padding does not refuse a call whose dense weights a memory limit allows.
+    const bool streams = adjoint_streams_weights(g) && !(g_mem_limit && scratch(gw) > g_mem_limit);
+    if (!streams) gw = g;
     const long long wn = (gw.cs + 63) / 64 * 64;
     char *base = nullptr;
-    int rc = grow(g_adj, 9 * (size_t) wn * sizeof(T) + 256, &base);
+    int rc = grow(g_adj, scratch(gw), &base);
     if (rc != DTB_OK) return rc;
     int dev = 0;
     DTB_CUDA(cudaGetDevice(&dev));

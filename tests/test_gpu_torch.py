@@ -304,3 +304,28 @@ def test_adjoint_keeps_infinities_local(shape, value):
                 assert torch.equal(~torch.isfinite(bad), reached)
                 assert torch.equal(bad[~reached], zero[~reached])
                 weight[place] = float(w[place])
+
+
+def test_adjoint_under_a_memory_limit():
+    """Odd widths pad their weights only where a memory limit has room for it:
+    20 x 21 x 45 needs 682240 bytes dense and 726016 padded."""
+    import torch
+
+    import disptools_b200 as dt
+    from disptools_b200 import _native as N
+    from disptools_b200 import torch_ops
+    rng = np.random.default_rng(5)
+    shape = (20, 21, 45)
+    field = torch.from_numpy(rng.normal(scale=0.2, size=(3,) + shape)).float().cuda()
+    weight = torch.from_numpy(rng.standard_normal(shape)).float().cuda()
+    want = torch_ops.jacobian_adjoint_raw(field, weight)
+    try:
+        N.check(N.lib.dtb_set_device_memory_limit(700000))
+        got = torch_ops.jacobian_adjoint_raw(field, weight)
+        N.check(N.lib.dtb_set_device_memory_limit(682239))
+        with pytest.raises(dt.DisptoolsError):
+            torch_ops.jacobian_adjoint_raw(field, weight)
+    finally:
+        N.check(N.lib.dtb_set_device_memory_limit(0))
+    # Thirteen terms a component, each rounded once in either order.
+    assert float((got - want).abs().max()) <= 13 * 2 ** -24 * 13 * float(want.abs().max())
