@@ -102,7 +102,7 @@ struct CentralWeights {
 // differences where `c4`, and are second order along every axis elsewhere
 // (schemes_at), one-sided where they lie on a face.
 template <int PX, int CELLS, typename TI, typename T>
-__device__ __forceinline__ void stencil_voxel(const TI *p, const TI (&zq)[3][5], int x, int y, int z, const Geom &g,
+__device__ __forceinline__ void stencil_voxel(const TI *p, const T (&zq)[3][5], int x, int y, int z, const Geom &g,
                                               const T (&ih)[3], bool deep, bool c4, T (&a)[3][3]) {
     auto central = [&](const CentralWeights<T> &w, auto second) {
 #pragma unroll
@@ -110,7 +110,7 @@ __device__ __forceinline__ void stencil_voxel(const TI *p, const TI (&zq)[3][5],
             const TI *q = p + c * CELLS;
             a[c][0] = w((T) q[1] - (T) q[-1], second((T) q[2] - (T) q[-2]), 0);
             a[c][1] = w((T) q[PX] - (T) q[-PX], second((T) q[2 * PX] - (T) q[-2 * PX]), 1);
-            a[c][2] = w((T) zq[c][3] - (T) zq[c][1], second((T) zq[c][4] - (T) zq[c][0]), 2);
+            a[c][2] = w(zq[c][3] - zq[c][1], second(zq[c][4] - zq[c][0]), 2);
         }
     };
     if (deep) {
@@ -207,11 +207,11 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
     const bool tile_in = TX == 32 && row_in && x0 >= 2 && x0 + L::X - 1 <= g.nx - 3;
     const bool voxel_in = row_in && x >= 2 && x <= g.nx - 3;
     const int own = (ty + 2) * L::PX + tx + 2;
-    TI zq[3][5];
+    T zq[3][5];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int k = 0; k < 5; ++k) zq[c][k] = TI(0);
+        for (int k = 0; k < 5; ++k) zq[c][k] = T(0);
     long long off = (z0 - 4) * g.zs + y * g.ys + x;  // of the thread's voxel in plane ze
     int slot = 0;                                    // of plane q
 #pragma unroll(sizeof(T) == 4 ? 5 : 1)
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(JA_NT, ja_blocks<T>())
         for (int c = 0; c < 3; ++c) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) zq[c][k] = zq[c][k + 1];
-            zq[c][4] = pl[c * L::CELLS];
+            zq[c][4] = (T) pl[c * L::CELLS];
         }
         const int ze = q - 2;
         const int se = slot >= 2 ? slot - 2 : slot - 2 + JA_NS;
