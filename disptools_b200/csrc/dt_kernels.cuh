@@ -65,9 +65,11 @@ __device__ __forceinline__ T det_i_plus(const T a[3][3]) {
 // ------------------------------------------------------------------------
 // FP32 pairs.  sm_100 executes add, sub, mul and fma on the two FP32 halves
 // of a 64-bit register pair as one instruction; each half rounds as the
-// scalar operation does.  The FP32 stencils below state every rounding
-// (no contraction left to the compiler), so the scalar and the paired forms
-// give the same bits for a voxel, whichever evaluator a tile takes.
+// scalar operation does.  The FP32 stencils below state every rounding.
+// ptxas still contracts a packed product with the packed sum or difference
+// that follows it (a scalar product marked _rn it leaves alone), so a paired
+// evaluator of products and sums can differ from the scalar one in the last
+// bit; which one a voxel takes depends on where it lies, not on the launch.
 // ------------------------------------------------------------------------
 __device__ __forceinline__ float2 p_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 p_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
@@ -137,11 +139,6 @@ __device__ __forceinline__ void schemes_at(int x, int y, int z, const Geom &g, i
         else
             k[a] = (g.order == 2 || pen) ? S_C2 : S_C4;
     }
-}
-
-__device__ __forceinline__ int ring_slot(int z, int ns) {
-    int s = z % ns;
-    return s < 0 ? s + ns : s;
 }
 
 // Per-voxel error of src/headers/error.h:128-142.

@@ -2690,7 +2690,7 @@ cudaError_t launch_gather_tma(const CUtensorMap &tm_wx, const CUtensorMap &tm_wy
 // Fused adjoint of the Jacobian map (autograd backward) with the TMA
 // pipeline: grad_c(q) = sum_a sum_t W[c][a](q - t e_a) kappa(k_a(q - t e_a), t)
 // with W[c][a](p) = gJ(p) cof_ca(I + A(p)) ih_a, A(p) the stencil matrix of
-// the Jacobian map at p (the two-pass path's k_adjoint_w / k_adjoint_gather),
+// the Jacobian map at p (the two-pass path's weights and gather),
 // without writing W to memory.
 //
 // A block of TXW / 2 x TYT threads marches a TXW x TT_Y tile through its z
