@@ -90,6 +90,12 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, u
         : "memory");
 }
 
+// Launches that overlap the end of the one before (see launch_step): waits
+// until the previous launch of the stream has finished and its writes are
+// visible; lets the next one's blocks start up to this wait.
+__device__ __forceinline__ void previous_launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_launch_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Per-thread asynchronous copy of one 4- or 8-byte element from global to
 // shared memory (cp.async, L1-allocating), grouped by commit and awaited by
 // the issuing thread only.
