@@ -329,3 +329,21 @@ def test_adjoint_under_a_memory_limit():
         N.check(N.lib.dtb_set_device_memory_limit(0))
     # Thirteen terms a component, each rounded once in either order.
     assert float((got - want).abs().max()) <= 13 * 2 ** -24 * 13 * float(want.abs().max())
+
+
+def test_backward_on_a_thread_without_a_context():
+    """The backward of a fresh process, its gradient's memory cached: the first
+    device work of the autograd thread."""
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "from disptools_b200 import torch_ops\n"
+            "f = 0.1 * torch.randn(3, 40, 40, 40, device='cuda')\n"
+            "w = torch.randn(40, 40, 40, device='cuda')\n"
+            "spare = [torch.empty_like(f) for _ in range(8)]\n"
+            "del spare\n"
+            "f.requires_grad_(True)\n"
+            "J = torch_ops.jacobian(f)\n"
+            "torch.autograd.grad(J, f, w)\n"
+            "torch.cuda.synchronize()\n")
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
