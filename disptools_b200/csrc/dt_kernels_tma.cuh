@@ -603,7 +603,9 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
         const bool stale_zero = GREEDY && (old_b == 0 || !ldcg_int(&st->b0_nonzero));
         const double eta = __ldcg(&st->eta);
         const T tol = (T) st->tolerance, delta = (T) st->delta, zeta = (T) st->zeta;
-        if (done) continue;
+        // A block that lost a transfer sets `done` at any time (tma_fault):
+        // the threads agree on what they read, so none goes on alone.
+        if (__syncthreads_or(done)) continue;
         const bool trial = phase != PH_EVAL0;
         const int lt = tile - V.tile_begin;
         const int txi = lt % V.tiles_x, tyi = (lt / V.tiles_x) % V.tiles_y, tzi = lt / (V.tiles_x * V.tiles_y);
@@ -987,7 +989,8 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
         SolverState *st = states + vol;
         const Geom g = V.g;
         const int done = ldcg_int(&st->done), wanted = ldcg_int(&st->need_gradient), old_b = ldcg_int(&st->old_buf);
-        if (done || !wanted) continue;
+        // Agreed on for the whole block, as in the trial kernel.
+        if (__syncthreads_or(done || !wanted)) continue;
         const int lt = tile - V.tile_begin;
         const int txi = lt % V.tiles_x, tyi = (lt / V.tiles_x) % V.tiles_y, tzi = lt / (V.tiles_x * V.tiles_y);
         const int x0 = txi * TXW, y0 = tyi * TT_Y, z0 = tzi * V.bz;

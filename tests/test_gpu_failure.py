@@ -137,3 +137,26 @@ def test_tiny_shapes_solver_fp64(oracle, shape):
         out, st = dt.solve(Jt, m, precision="fp64", algorithm=alg, it_max=30)
         assert st["iterations"] == so.iterations and st["reason"] == so.reason
         assert np.max(np.abs(out - ref)) <= 1e-10
+
+
+@pytest.mark.parametrize("algorithm", ["gradient", "greedy"])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_dropped_load_while_blocks_take_tiles(precision, algorithm, monkeypatch):
+    """576 tiles on at most 296 blocks: the volume is marked as failed while
+    other blocks read its state for their next tile.  A block takes that tile
+    as a whole or not at all, the solve ends with the error, every time, and
+    the device is as good as before."""
+    monkeypatch.setenv("DISPTOOLS_B200_BZ", "3")
+    Jt, m = ball_problem(96, 48, 20, 1.1)
+    kw = dict(precision=precision, algorithm=algorithm, it_max=4)
+    good, sg = dt.solve(Jt, m, **kw)
+    try:
+        for tile, iteration in ((0, 1), (17, 3), (150, 6), (300, 0), (575, 2)):
+            N.check(N.lib.dtb_test_drop_tma_load(tile, iteration, 1 << 10))
+            with pytest.raises(dt.DisptoolsError, match="did not complete within its bound"):
+                dt.solve(Jt, m, **kw)
+    finally:
+        N.check(N.lib.dtb_test_drop_tma_load(-1, -1, 0))
+    again, sa = dt.solve(Jt, m, **kw)
+    np.testing.assert_array_equal(good, again)
+    assert sg["trials"] == sa["trials"]
