@@ -118,6 +118,16 @@ struct GradTmaLayout {
     static constexpr int BYTES = BAR_OFF + S * 8;
 };
 
+// Counts a block out of a launch; the last one resets the queue for the next.
+__device__ __forceinline__ void leave_queue(TileQueue *q) {
+    __threadfence();
+    if (atomicAdd(&q->exited, 1u) == gridDim.x - 1) {
+        q->next = 0;
+        q->exited = 0;
+        __threadfence();
+    }
+}
+
 // Takes the next tile of a persistent launch (-1 when none is left; the
 // block is then counted out and the last one resets the queue).  A block's
 // first tile is its own number, without the queue's round trip.  BDX is the
@@ -130,12 +140,7 @@ __device__ __forceinline__ int take_tile(TileQueue *q, int total, int *s_tile) {
         int t = (int) (gridDim.x + atomicAdd(&q->next, 1u));
         if (t >= total) {
             t = -1;
-            __threadfence();
-            if (atomicAdd(&q->exited, 1u) == gridDim.x - 1) {
-                q->next = 0;
-                q->exited = 0;
-                __threadfence();
-            }
+            leave_queue(q);
         }
         *s_tile = t;
     }
@@ -895,7 +900,10 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
         }
         if (failed) {
             if (GREEDY) cp_async_wait_all();  // no element copy lands after the block has left
-            if (tid == 0) tma_fault<L::S>(st, bars, kbase, fail_it + 1, issued_n);
+            if (tid == 0) {
+                tma_fault<L::S>(st, bars, kbase, fail_it + 1, issued_n);
+                leave_queue(queue);
+            }
             __syncthreads();
             return;
         }
@@ -1303,7 +1311,10 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
             ps = ps + 1 < L::NP ? ps + 1 : 0;
         }
         if (failed) {
-            if (tid == 0) tma_fault<L::S>(st, bars, kbase, fail_it + 1, issued_n);
+            if (tid == 0) {
+                tma_fault<L::S>(st, bars, kbase, fail_it + 1, issued_n);
+                leave_queue(queue);
+            }
             __syncthreads();
             return;
         }
@@ -1729,6 +1740,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                     const uint32_t kk = kbase + j;
                     mbar_wait_bounded(&bars[kk % S], (kk / S) & 1u, 1u << 16);
                 }
+                leave_queue(queue);
             }
             __syncthreads();
             return;

@@ -160,3 +160,29 @@ def test_dropped_load_while_blocks_take_tiles(precision, algorithm, monkeypatch)
     again, sa = dt.solve(Jt, m, **kw)
     np.testing.assert_array_equal(good, again)
     assert sg["trials"] == sa["trials"]
+
+
+@pytest.mark.parametrize("volume", [0, 1])
+@pytest.mark.parametrize("algorithm,trial_kernel", [("gradient", "formed"), ("gradient", "release"),
+                                                    ("greedy", "formed")])
+def test_dropped_load_in_a_batch(algorithm, trial_kernel, volume, monkeypatch):
+    """The block that lost its transfer leaves the launch counted, so the
+    other volume's solve takes each of its tiles once a launch and comes to
+    its end: the error is the lost transfer's, not a solve without end."""
+    monkeypatch.setenv("DISPTOOLS_B200_TRIAL_KERNEL", trial_kernel)
+    monkeypatch.setenv("DISPTOOLS_B200_BZ", "3")
+    problems = [ball_problem(n, n / 2, n / 4, 1.1) for n in (72, 64)]
+    kw = dict(algorithm=algorithm, precision="mixed", it_max=6)
+    good = dt.solve_batched(problems, **kw)
+    tile = 5 if volume == 0 else (-(-72 // 32)) * (-(-72 // 16)) * (72 // 3) + 5
+    N.check(N.lib.dtb_test_drop_tma_load(tile, 2, 1 << 10))
+    try:
+        for _ in range(3):
+            with pytest.raises(dt.DisptoolsError, match="did not complete within its bound"):
+                dt.solve_batched(problems, **kw)
+    finally:
+        N.check(N.lib.dtb_test_drop_tma_load(-1, -1, 0))
+    again = dt.solve_batched(problems, **kw)
+    for (a, sa), (b, sb) in zip(good, again):
+        np.testing.assert_array_equal(a, b)
+        assert sa["trials"] == sb["trials"]
