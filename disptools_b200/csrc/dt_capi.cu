@@ -378,16 +378,19 @@ int num_sms() {
 
 // Per-device resources that live across solves: the solver's own stream,
 // pinned host mirrors, events and the captured step graph (reused while the
-// launch configuration is unchanged).
+// launch configuration is unchanged).  The key has every pointer and size that
+// the captured launches hold: after the workspace has moved, no part of one
+// layout may come with another of an old one.
 struct GraphKey {
     size_t tsize = 0;
     int algorithm = -1;
-    const void *desc = nullptr;
-    const int *tile_vol = nullptr;
+    const void *desc = nullptr, *states = nullptr, *queues = nullptr;
+    const int *tile_vol = nullptr;  // null: one volume
     int total_tiles = 0, grid_t = 0, grid_g = 0, grid_b = 0, K = 0, threads_y = 0;
     const unsigned char *flags = nullptr;
     bool operator==(const GraphKey &o) const {
-        return tsize == o.tsize && algorithm == o.algorithm && desc == o.desc && tile_vol == o.tile_vol &&
+        return tsize == o.tsize && algorithm == o.algorithm && desc == o.desc && states == o.states &&
+               queues == o.queues && tile_vol == o.tile_vol &&
                total_tiles == o.total_tiles && grid_t == o.grid_t && grid_g == o.grid_g && grid_b == o.grid_b &&
                K == o.K && threads_y == o.threads_y && flags == o.flags;
     }
@@ -815,7 +818,9 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
     key.tsize = sizeof(T);
     key.algorithm = algorithm;
     key.desc = d_desc;
-    key.tile_vol = d_tile_vol;
+    key.states = d_state0;
+    key.queues = d_queues;
+    key.tile_vol = rel ? d_tile_vol : tv;
     key.total_tiles = total_tiles;
     key.grid_t = grid_t;
     key.grid_g = grid_g;

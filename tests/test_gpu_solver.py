@@ -474,3 +474,24 @@ def test_host_arrays_through_staging(shape):
     with ThreadPoolExecutor(3) as pool:
         for got in pool.map(api.jacobian, [field] * 6):
             np.testing.assert_array_equal(got, map_want)
+
+
+@pytest.mark.parametrize("algorithm", ["gradient", "greedy"])
+def test_results_as_the_workspace_grows(algorithm):
+    """Solves of growing and shrinking layouts, one volume and several, each
+    after the workspace has moved or the step graph of another layout was
+    kept: each the field of the same solve on a fresh workspace."""
+    rng = np.random.default_rng(11)
+    shapes = [[(8, 9, 10)], [(8, 9, 26)], [(8, 9, 10)] * 2, [(20, 33, 17)], [(8, 9, 10)], [(40, 41, 42), (8, 9, 10)],
+              [(20, 33, 17)], [(48, 50, 70)], [(8, 9, 26)], [(8, 9, 10)] * 2]
+    problems = [[(1.0 + 0.05 * rng.standard_normal(s), rng.random(s) < 0.5) for s in group] for group in shapes]
+    kw = dict(algorithm=algorithm, precision="fp64", it_max=8)
+    fresh = []
+    for group in problems:
+        dt.release_device_memory()
+        fresh.append(dt.solve_batched(group, **kw))
+    dt.release_device_memory()
+    for group, want in zip(problems, fresh):
+        for (a, sa), (b, sb) in zip(dt.solve_batched(group, **kw), want):
+            np.testing.assert_array_equal(a, b)
+            assert sa["trials"] == sb["trials"]
