@@ -575,7 +575,7 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
     // ---- workspace layout: every buffer of the solve is the library's own,
     // in the pitched layout.
     const long long log_cap = (verbose_enabled() && !tune_ms)
-                                  ? std::min<long long>(4 * (std::max<long long>(p.it_max, 0) + 16), 1ll << 20)
+                                  ? std::min<long long>(4 * (std::clamp<long long>(p.it_max, 0, 1ll << 20) + 16), 1ll << 20)
                                   : 0;
     std::vector<int> tiles(count), tbegin(count);
     std::vector<Geom> geo(count);
@@ -878,8 +878,8 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
     // its launches.
     rc = ensure_host_states(e, count);
     if (rc != DTB_OK) return rc;
-    long long max_steps = 0;
-    for (int i = 0; i < count; ++i) max_steps = std::max(max_steps, 64 * (p.it_max + 2) + 4096);
+    // 64 trials an iteration; a limit far beyond reach ("none") must not wrap.
+    const long long max_steps = 64 * (std::min(p.it_max, (LLONG_MAX - 4096) / 64 - 2) + 2) + 4096;
     long long steps = 0;
     int status = DTB_OK;
     cudaError_t loop_err = cudaSuccess;

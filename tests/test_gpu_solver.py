@@ -495,3 +495,24 @@ def test_results_as_the_workspace_grows(algorithm):
         for (a, sa), (b, sb) in zip(dt.solve_batched(group, **kw), want):
             np.testing.assert_array_equal(a, b)
             assert sa["trials"] == sb["trials"]
+
+
+@pytest.mark.parametrize("algorithm", ["gradient", "greedy"])
+def test_any_iteration_limit(algorithm, capfd):
+    """A limit far beyond reach ("no limit") is the same as one just out of
+    reach: neither the bound on queued steps nor the size of the verbose log
+    wraps."""
+    Jt, m = ball_problem(24, 12, 6, 1.1)
+    kw = dict(algorithm=algorithm, precision="fp64", epsilon=0.02)
+    want, sw = dt.solve(Jt, m, it_max=100000, **kw)
+    assert 16 < sw["trials"] and sw["iterations"] < 100000
+    for it_max in (2 ** 57, 2 ** 62, 2 ** 63 - 1):
+        for verbose in (False, True):
+            before = dt.set_verbose(verbose)
+            try:
+                got, sg = dt.solve(Jt, m, it_max=it_max, **kw)
+            finally:
+                dt.set_verbose(before)
+            assert sg["iterations"] == sw["iterations"]
+            np.testing.assert_array_equal(got, want)
+            assert capfd.readouterr().out.count("Iteration ") >= (sw["iterations"] if verbose else 0)
