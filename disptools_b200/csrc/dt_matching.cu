@@ -868,8 +868,9 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
         M_CUDA(cudaEventRecord(ev.e[3 + (r & 1)], s));
         return DTB_OK;
     };
-    // An iteration's doublings and halvings span the float range at most.
-    const long long max_steps = 400 * (std::max<long long>(p.it_max, 0) + 2);
+    // An iteration's doublings and halvings span the float range at most.  A
+    // limit far beyond reach ("none") must not wrap.
+    const long long max_steps = 400 * (std::clamp<long long>(p.it_max, 0, LLONG_MAX / 400 - 2) + 2);
     MatchState last = init;
     auto run = [&]() -> int {
         int rc = enqueue(0);

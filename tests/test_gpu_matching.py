@@ -182,3 +182,16 @@ def test_device_step_control_against_float64(target, delta, zeta, wanted):
     z, y, x = np.meshgrid(*[np.arange(1, n + 1) for n in J.shape], indexing="ij")
     ref = np.stack([pos[1].numpy() - x, pos[0].numpy() - y, pos[2].numpy() - z])
     assert np.max(np.abs(out - ref)) <= 1e-4
+
+
+@pytest.mark.parametrize("it_max", [2 ** 56, 2 ** 62, 2 ** 63 - 1])
+def test_matching_takes_any_iteration_limit(it_max):
+    """A limit far beyond reach ("no limit") is the same as one just out of
+    reach: the bound on queued steps does not wrap."""
+    Jt, m = ball_problem(16, 8, 4, 1.1)
+    kw = dict(algorithm="matching", epsilon=0.02)
+    want, sw = dt.solve(Jt, m, it_max=100000, **kw)
+    assert 16 < sw["iterations"] < 100000
+    got, sg = dt.solve(Jt, m, it_max=it_max, **kw)
+    assert sg["iterations"] == sw["iterations"]
+    np.testing.assert_array_equal(got, want)
