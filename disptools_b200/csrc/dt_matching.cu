@@ -791,10 +791,12 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
     // Gradient: two blocks fit on an SM and each run also forms the layer below
     // it, so the depth whose busiest SM has least to do; a block alone on its
     // SM runs about 1.5 times as fast as one of two.  At 96^3 runs of 16 layers
-    // (two blocks an SM) take 42.9 us, runs of 4 (eight) 49.6 us.
-    int zc_grad = 1;
+    // (two blocks an SM) take 42.9 us, runs of 4 (eight) 49.6 us.  No shorter
+    // than a grid has room for along z.
+    const int zc_min = ((int) nz + 65534) / 65535;
+    int zc_grad = zc_min;
     double best = 1e300;
-    for (int zc = std::min((int) nz, 64); zc >= 1; --zc) {
+    for (int zc = std::min((int) nz, std::max(64, zc_min)); zc >= zc_min; --zc) {
         const long long q = (grad_tiles * (((int) nz + zc - 1) / zc) + 147) / 148;
         const double t = (zc + 2) * ((double) (q / 2 * 2) + (q % 2 ? 1.3 : 0.0));
         if (t < best) {

@@ -195,3 +195,25 @@ def test_matching_takes_any_iteration_limit(it_max):
     got, sg = dt.solve(Jt, m, it_max=it_max, **kw)
     assert sg["iterations"] == sw["iterations"]
     np.testing.assert_array_equal(got, want)
+
+
+def test_matching_of_a_long_column():
+    """2 x 2 x 4.3 million voxels, more gradient runs than a grid has z blocks:
+    away from the one place that moves nothing does, so the first planes are
+    those of the short column (only the cost's summation order differs)."""
+    import torch
+
+    from disptools_b200 import torch_ops
+    results = []
+    for nz in (400, 4_300_000):
+        J = torch.ones((nz, 2, 2), dtype=torch.float64, device="cuda")
+        J[40:60] = 1.05
+        field = torch.zeros((3, nz, 2, 2), dtype=torch.float64, device="cuda")
+        st = torch_ops.solve(J, torch.ones(J.shape, dtype=torch.bool, device="cuda"), field, algorithm="matching",
+                             it_max=4)
+        results.append((field, st["iterations"]))
+    (short, it_short), (long, it_long) = results
+    assert it_long == it_short > 0
+    assert float(short.abs().max()) > 0.0
+    torch.testing.assert_close(long[:, :300], short[:, :300], rtol=0, atol=1e-5)
+    assert not long[:, 300:].any()
