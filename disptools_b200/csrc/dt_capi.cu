@@ -493,6 +493,7 @@ bool verbose_enabled() {
 // The greedy method runs 32 x TT_Y tiles of bz planes.
 struct TileConfig {
     int tile_x = 32, trial_ty = 16, grad_ty = 16, bz = 32, pf = 0, trial_kind = 0;
+    bool depth_by_model = false;  // bz from wave_filled_bz, not from a caller or a list
 };
 
 // Explicit shapes from the environment (DISPTOOLS_B200_TILE_X = 32 | 64,
@@ -562,11 +563,6 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
         const int rc0 = choose_config<T>(e, algorithm, vols, p, precision, &cfg);
         if (rc0 != DTB_OK) return rc0;
     }
-    e->last_cfg[0] = cfg.tile_x;
-    e->last_cfg[1] = cfg.trial_ty;
-    e->last_cfg[2] = cfg.grad_ty;
-    e->last_cfg[3] = cfg.bz;
-    e->last_trial_kind = cfg.trial_kind;
     // The greedy trial kernel exists for 32-wide tiles only.
     const int tile_x = algorithm == DTB_ALGORITHM_GRADIENT ? cfg.tile_x : 32;
     const int threads_y = cfg.grad_ty;
@@ -580,27 +576,43 @@ int solve_device_on(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols
     std::vector<int> tiles(count), tbegin(count);
     std::vector<Geom> geo(count);
     int total_tiles = 0;
-    size_t need = 0;
     auto align = [](size_t b) { return (b + 255) & ~size_t(255); };
     const int tile_y = TT_Y;
-    for (int i = 0; i < count; ++i) {
-        const Geom g = pitched(vols[i].g);
-        geo[i] = g;
-        const int bz = bz_for(g.nz, cfg.bz);
-        const int t = ((g.nx + tile_x - 1) / tile_x) * ((g.ny + tile_y - 1) / tile_y) * ((g.nz + bz - 1) / bz);
-        tiles[i] = t;
-        tbegin[i] = total_tiles;
-        total_tiles += t;
-        const size_t N = (size_t) g.cs;
-        need += 3 * align(3 * N * sizeof(T));       // field[0], field[1], gradient
-        need += align(N * sizeof(T)) + align(N);     // target map, mask
-        need += 2 * align(N * sizeof(T));            // e' (gradient) or error maps (greedy)
-        need += align(t * sizeof(double2)) + align(t * sizeof(double));
-        need += align(7 * sizeof(CUtensorMap));
-        need += align((size_t) log_cap * sizeof(IterLog));
+    // Tiles of cfg.bz planes and the bytes that they and the volumes need.
+    auto lay_out = [&]() -> size_t {
+        total_tiles = 0;
+        size_t need = 0;
+        for (int i = 0; i < count; ++i) {
+            const Geom g = pitched(vols[i].g);
+            geo[i] = g;
+            const int bz = bz_for(g.nz, cfg.bz);
+            const int t = ((g.nx + tile_x - 1) / tile_x) * ((g.ny + tile_y - 1) / tile_y) * ((g.nz + bz - 1) / bz);
+            tiles[i] = t;
+            tbegin[i] = total_tiles;
+            total_tiles += t;
+            const size_t N = (size_t) g.cs;
+            need += 3 * align(3 * N * sizeof(T));       // field[0], field[1], gradient
+            need += align(N * sizeof(T)) + align(N);     // target map, mask
+            need += 2 * align(N * sizeof(T));            // e' (gradient) or error maps (greedy)
+            need += align(t * sizeof(double2)) + align(t * sizeof(double));
+            need += align(7 * sizeof(CUtensorMap));
+            need += align((size_t) log_cap * sizeof(IterLog));
+        }
+        return need + align(count * sizeof(VolumeDesc<T>)) + align(total_tiles * sizeof(int)) +
+               align(2 * sizeof(TileQueue)) + align(count * sizeof(SolverState));
+    };
+    size_t need = lay_out();
+    // The partial sums of thin tiles do not refuse a solve that a memory limit
+    // allows at the default depth.
+    if (cfg.depth_by_model && g_mem_limit && need > g_mem_limit) {
+        cfg.bz = std::max(cfg.bz, TileConfig().bz);
+        need = lay_out();
     }
-    need += align(count * sizeof(VolumeDesc<T>)) + align(total_tiles * sizeof(int)) + align(2 * sizeof(TileQueue)) +
-            align(count * sizeof(SolverState));
+    e->last_cfg[0] = cfg.tile_x;
+    e->last_cfg[1] = cfg.trial_ty;
+    e->last_cfg[2] = cfg.grad_ty;
+    e->last_cfg[3] = cfg.bz;
+    e->last_trial_kind = cfg.trial_kind;
 
     char *base = nullptr;
     int rc = workspace(need, &base);
@@ -1115,13 +1127,13 @@ std::vector<TileConfig> tile_candidates(size_t tsize, int bzw, int bzd) {
     std::vector<TileConfig> c;
     auto listed = [](int bz) { return bz == 16 || bz == 32 || bz == 64; };
     const bool wave = !listed(bzw);
-    if (wave) c.push_back({32, 16, 16, bzw});
-    if (bzd != bzw && !listed(bzd)) c.push_back({32, 16, 16, bzd});
+    if (wave) c.push_back({32, 16, 16, bzw, 0, 0, true});
+    if (bzd != bzw && !listed(bzd)) c.push_back({32, 16, 16, bzd, 0, 0, true});
     const std::vector<TileConfig> fixed = {{32, 16, 16, 32}, {32, 16, 8, 32}, {32, 16, 16, 16}, {32, 16, 16, 64},
                                            {32, 8, 16, 32}};
     c.insert(c.end(), fixed.begin(), fixed.end());
     if (tsize == 4) c.push_back({64, 16, 8, 32});
-    if (wave) c.push_back({32, 16, 8, bzw});
+    if (wave) c.push_back({32, 16, 8, bzw, 0, 0, true});
     // The trial kernel without the per-plane barrier (trial_kind 1) is not a
     // candidate: at 256^3 it took 0.305-0.315 ms a launch against 0.227-0.233
     // ms for the formed-plane kernel.  The environment can still select it.
@@ -1150,6 +1162,7 @@ int choose_config(Engine *e, int algorithm, const std::vector<DevVol<T>> &vols, 
     }
     if (!gradient || key.voxels < AUTOTUNE_MIN_VOXELS || !autotune_enabled()) {
         c.bz = wave_filled_bz(geo, 32, slots, 2, 32);
+        c.depth_by_model = true;
         *out = c;
         return DTB_OK;
     }

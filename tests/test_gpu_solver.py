@@ -516,3 +516,42 @@ def test_any_iteration_limit(algorithm, capfd):
             assert sg["iterations"] == sw["iterations"]
             np.testing.assert_array_equal(got, want)
             assert capfd.readouterr().out.count("Iteration ") >= (sw["iterations"] if verbose else 0)
+
+
+@pytest.mark.parametrize("algorithm", ["gradient", "greedy"])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_thin_tiles_give_way_to_a_memory_limit(monkeypatch, algorithm, precision):
+    """A limit that is just enough for 32-plane tiles is enough for the depth
+    the solve picks by itself, whose partial sums take more room."""
+    from disptools_b200 import _native as N
+    Jt, m = ball_problem(40, 20, 9, 1.1)
+    kw = dict(algorithm=algorithm, precision=precision, it_max=3)
+
+    def solves(limit):
+        dt.release_device_memory()
+        N.check(N.lib.dtb_set_device_memory_limit(limit))
+        try:
+            return dt.solve(Jt, m, **kw)[0]
+        except dt.DisptoolsError:
+            return None
+        finally:
+            N.check(N.lib.dtb_set_device_memory_limit(0))
+
+    monkeypatch.setenv("DISPTOOLS_B200_BZ", "32")
+    lo, hi = 1 << 20, 1 << 26  # refused, enough
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        if solves(mid) is None:
+            lo = mid
+        else:
+            hi = mid
+    deep = solves(hi)
+    assert deep is not None and solves(hi - 1) is None
+    monkeypatch.delenv("DISPTOOLS_B200_BZ")
+    got = solves(hi)
+    assert got is not None
+    np.testing.assert_array_equal(got, deep)
+    assert solves(hi - 1) is None
+    # An explicit depth is not changed.
+    monkeypatch.setenv("DISPTOOLS_B200_BZ", "2")
+    assert solves(hi) is None
