@@ -1526,12 +1526,21 @@ int adjoint_device_impl(const Geom &g, const T *field, const T *gJ, T *gout, cud
     gw.ys = (g.nx + v - 1) / v * v;
     gw.zs = gw.ys * g.ny;
     gw.cs = gw.zs * g.nz;
-    // Padding does not refuse a call whose dense weights a memory limit allows.
-    const bool streams = adjoint_streams_weights(g) && !(g_mem_limit && scratch(gw) > g_mem_limit);
-    if (!streams) gw = g;
-    const long long wn = (gw.cs + 63) / 64 * 64;
+    bool streams = adjoint_streams_weights(g);
+    long long wn = 0;
     char *base = nullptr;
-    int rc = grow(g_adj, scratch(gw), &base);
+    auto take = [&](const Geom &w) -> int {
+        gw = w;
+        wn = (gw.cs + 63) / 64 * 64;
+        return grow(g_adj, scratch(gw), &base);
+    };
+    int rc = take(streams ? gw : g);
+    if (rc == DTB_ERR_ALLOC && streams) {
+        // Padding does not refuse a call whose dense weights fit.
+        disptools_clear_error();
+        streams = false;
+        rc = take(g);
+    }
     if (rc != DTB_OK) return rc;
     int dev = 0;
     DTB_CUDA(cudaGetDevice(&dev));
@@ -1543,21 +1552,23 @@ int adjoint_device_impl(const Geom &g, const T *field, const T *gJ, T *gout, cud
     // allows it (as for the Jacobian map), else on the element-wise kernel.
     const CUtensorMapDataType ft = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
     CUtensorMap tm, tw[3];
+    if (streams && !(encode_weights_map(&tw[0], ft, sizeof(T), W, gw, wn, 32 + 2 * 4, TT_Y) &&
+                     encode_weights_map(&tw[1], ft, sizeof(T), W, gw, wn, 32, TT_Y + 2 * 2) &&
+                     encode_weights_map(&tw[2], ft, sizeof(T), W, gw, wn, 32, TT_Y))) {
+        streams = false;
+        rc = take(g);  // dense weights need no more room
+        if (rc != DTB_OK) return rc;
+    }
     if (tma_stencil_pays<T>(g) && g.order == 4 && (g.ys * (long long) sizeof(T)) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(field) % 16 == 0 && reinterpret_cast<uintptr_t>(gJ) % (2 * sizeof(T)) == 0 &&
         encode_map(&tm, ft, sizeof(T), field, g, 3, 32 + 2 * 4, TT_Y + 2 * 2))
         DTB_CUDA(launch_jacobian_tma<T>(tm, g, nullptr, g.ys, g.zs, num_sms(), s, gJ, W, wn));
     else
         DTB_CUDA(launch_weights_any<T>(field, g, gJ, W, wn, gw.ys, gw.zs, num_sms(), s));
-    if (streams) {
-        if (!(encode_weights_map(&tw[0], ft, sizeof(T), W, gw, wn, 32 + 2 * 4, TT_Y) &&
-              encode_weights_map(&tw[1], ft, sizeof(T), W, gw, wn, 32, TT_Y + 2 * 2) &&
-              encode_weights_map(&tw[2], ft, sizeof(T), W, gw, wn, 32, TT_Y)))
-            DTB_FAIL(DTB_ERR_CUDA, "cannot encode the TMA descriptors (cuTensorMapEncodeTiled)");
+    if (streams)
         DTB_CUDA(launch_gather_tma<T>(tw[0], tw[1], tw[2], g, gout, num_sms(), s));
-    } else {
+    else
         DTB_CUDA(launch_adjoint_gather<T>(g, W, wn, gout, s));
-    }
     DTB_CUDA(cudaEventRecord(g_adj_done[dev], s));
     return DTB_OK;
 }
