@@ -1792,9 +1792,9 @@ cudaError_t launch_step(void (*kernel)(P...), bool early, int grid, dim3 block, 
     config.stream = s;
     config.attrs = &attr;
     config.numAttrs = early ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, P(args)...);
+    cudaLaunchKernelEx(&config, kernel, P(args)...);
     count_launch();
-    return e;
+    return cudaGetLastError();
 }
 
 template <typename T, int TXW, int TYT>
