@@ -729,6 +729,14 @@ private:
     }
 };
 
+// Waits for the stream's work at the end of its scope, whichever way that ends.
+struct StreamEnd {
+    cudaStream_t s;
+    ~StreamEnd() {
+        if (cudaStreamSynchronize(s) != cudaSuccess) cudaGetLastError();
+    }
+};
+
 // Events, destroyed with the object: three for timing, two that follow a batch.
 struct Events {
     cudaEvent_t e[5] = {};
@@ -820,6 +828,7 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
         report(__LINE__, __func__, "cannot allocate device buffers");
         return DTB_ERR_ALLOC;
     }
+    const StreamEnd end{s};  // goes first, so nothing is in flight when the others go
     float *const pos[2] = {b.at<float>(o_pos0), b.at<float>(o_pos1)}, *const step = b.at<float>(o_step);
     float *const tv = b.at<float>(o_tv);
     double2 *const partial = b.at<double2>(o_partial);
@@ -898,11 +907,7 @@ int matching_solve(size_t nx, size_t ny, size_t nz, double dx, double dy, double
         }
     };
     const int rc = run();
-    if (rc != DTB_OK) {
-        cudaStreamSynchronize(s);  // before the memory goes
-        cudaGetLastError();
-        return rc;
-    }
+    if (rc != DTB_OK) return rc;
 
     // Back to displacements in the caller's layout (:777-787).
     float *const cur = pos[last.cur];
