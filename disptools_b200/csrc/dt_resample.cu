@@ -34,6 +34,7 @@
 //   into the volume.  Nearest mode takes floor(p + 0.5).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -272,16 +273,6 @@ __device__ __forceinline__ double lerp_rn(double a, double b, double f) {
     return __dadd_rn(a, __dmul_rn(__dsub_rn(b, a), f));
 }
 
-// A block of 32 x 8 threads takes 32 x 8 output columns and RS_Z output planes
-// of every component.  Its sample places are divided for once, into shared
-// memory, and a thread keeps the two input planes it has interpolated along x
-// and y while the output planes lie between them: towards a finer grid that is
-// half an input plane per output plane instead of two.  (One thread per voxel,
-// with its three divisions and 64-bit index arithmetic, took 3.46 ms for three
-// FP32 components of 384 x 512 x 512 from half the size; places once per
-// thread and no planes kept, 1.91 ms.)
-constexpr int RS_X = 32, RS_Y = 8, RS_Z = 16;
-
 struct SamplePlace {
     double f;      // weight of the upper neighbour
     int i0, i1;    // neighbours in the volume; both the nearest sample in nearest mode
@@ -302,6 +293,63 @@ __device__ __forceinline__ SamplePlace sample_place(int i2, int n, int n2, int m
     }
     return a;
 }
+
+// One thread per output voxel and component: the kernel of outputs that the
+// tiles below do not serve (tiles_serve).
+template <typename T>
+__global__ void k_resample_voxel(const T *__restrict__ in, T *__restrict__ out, int nx, int ny, int nz, int nx2,
+                                 int ny2, int nz2, int comps, int mode) {
+    const long long n2 = (long long) nx2 * ny2 * nz2 * comps;
+    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n2;
+         i += (long long) gridDim.x * blockDim.x) {
+        const int x2 = (int) (i % nx2);
+        long long r = i / nx2;
+        const int y2 = (int) (r % ny2);
+        r /= ny2;
+        const int z2 = (int) (r % nz2);
+        const int c = (int) (r / nz2);
+        const double px = __ddiv_rn((double) x2 * (double) nx, (double) nx2);
+        const double py = __ddiv_rn((double) y2 * (double) ny, (double) ny2);
+        const double pz = __ddiv_rn((double) z2 * (double) nz, (double) nz2);
+        const bool inside = px >= -0.5 && px < nx - 0.5 && py >= -0.5 && py < ny - 0.5 && pz >= -0.5 &&
+                            pz < nz - 0.5;
+        if (!inside) {
+            out[i] = T(0);
+            continue;
+        }
+        const T *vol = in + (long long) c * nx * ny * nz;
+        auto at = [&](int x, int y, int z) -> double {
+            return (double) vol[((long long) z * ny + y) * nx + x];
+        };
+        if (mode == DTB_RESAMPLE_NEAREST) {
+            const int x = min((int) floor(px + 0.5), nx - 1);
+            const int y = min((int) floor(py + 0.5), ny - 1);
+            const int z = min((int) floor(pz + 0.5), nz - 1);
+            out[i] = (T) at(x, y, z);
+            continue;
+        }
+        const double fx0 = floor(px), fy0 = floor(py), fz0 = floor(pz);
+        const double fx = __dsub_rn(px, fx0), fy = __dsub_rn(py, fy0), fz = __dsub_rn(pz, fz0);
+        const int x0 = max((int) fx0, 0), y0 = max((int) fy0, 0), z0 = max((int) fz0, 0);
+        const int x1 = min((int) fx0 + 1, nx - 1), y1 = min((int) fy0 + 1, ny - 1), z1 = min((int) fz0 + 1, nz - 1);
+        const double c00 = lerp_rn(at(x0, y0, z0), at(x1, y0, z0), fx);
+        const double c10 = lerp_rn(at(x0, y1, z0), at(x1, y1, z0), fx);
+        const double c01 = lerp_rn(at(x0, y0, z1), at(x1, y0, z1), fx);
+        const double c11 = lerp_rn(at(x0, y1, z1), at(x1, y1, z1), fx);
+        const double c0 = lerp_rn(c00, c10, fy);
+        const double c1 = lerp_rn(c01, c11, fy);
+        out[i] = (T) lerp_rn(c0, c1, fz);
+    }
+}
+
+// A block of 32 x 8 threads takes 32 x 8 output columns and RS_Z output planes
+// of every component.  Its sample places are divided for once, into shared
+// memory, and a thread keeps the two input planes it has interpolated along x
+// and y while the output planes lie between them: towards a finer grid that is
+// half an input plane per output plane instead of two.  Three FP32 components
+// of 384 x 512 x 512 from half the size take 0.69 ms, one thread per voxel 3.46
+// ms; places once per thread and no planes kept, 1.91 ms.
+constexpr int RS_X = 32, RS_Y = 8, RS_Z = 16;
 
 template <typename T>
 __global__ void __launch_bounds__(RS_X *RS_Y)
@@ -467,6 +515,58 @@ cudaError_t smooth(int comps, int nx, int ny, int nz, const SmoothWeights (&sw)[
     return cudaGetLastError();
 }
 
+// Blocks of the tile kernel.
+long long resample_tiles(const int (&to)[3]) {
+    return ((long long) to[0] + RS_X - 1) / RS_X * (((long long) to[1] + RS_Y - 1) / RS_Y) *
+           (((long long) to[2] + RS_Z - 1) / RS_Z);
+}
+
+// Whether tiles (k_resample) or single voxels (k_resample_voxel) are faster, by
+// estimates in us.  A tile is a chain: its planes and components one after the
+// other, each with as many interpolated input planes as the ratio along z asks
+// for.  So a few tiles take as long as one (15 us for three components towards a
+// finer grid, 30 towards a coarser one), lanes beyond a narrow row idle, and
+// towards a coarser grid no plane is used twice.  Constants fitted to both
+// kernels' times at 660 shapes from 8^3 to 1.5e7 voxels, widths from 1, ratios
+// 1/4 to 4, one and three components, both types and modes; the faster one is
+// taken but for 1 % of time on average (tiles always: 44 %, voxels 31 %).  Three
+// FP32 components, linear, us by tiles and by voxels: 32^3 to 64^3 15 and 15, 48^3
+// to 96^3 17 and 37, 128^3 to 256^3 123 and 587; 64^3 to 32^3 29 and 5, 192^3 to
+// 96^3 57 and 39, 384^3 to 192^3 163 and 263; 2000 x 2000 x 1 from half 757 and 178.
+bool tiles_serve(int mode, int comps, const int (&from)[3], const int (&to)[3]) {
+    const double tiles = (double) resample_tiles(to);
+    if (tiles > INT_MAX) return false;
+    const double ratio = (double) from[2] / to[2];
+    const double columns = (double) ((to[0] + RS_X - 1) / RS_X);
+    const double warp_planes = columns * to[1] * to[2] * comps;
+    const double chain = comps * (double) std::min(RS_Z, to[2]);
+    double tile_us, voxel_us;
+    if (mode == DTB_RESAMPLE_NEAREST) {
+        tile_us = 3.5 + std::hypot(chain * 0.23, warp_planes * 0.61e-4) + tiles * 1.8e-3;
+        voxel_us = 3.0 + 1.06e-5 * to[0] * (double) to[1] * to[2] * comps;
+    } else {
+        const double s = std::min(ratio, 2.0);
+        tile_us = 3.5 + std::hypot(chain * (0.13 + 0.24 * s), warp_planes * (0.12e-4 + 0.99e-4 * s)) + tiles * 2.2e-3;
+        voxel_us = 3.0 + 1.45e-5 * to[0] * (double) to[1] * to[2] * comps;
+    }
+    // Towards a coarser grid a tile's reads scatter further than the estimate
+    // knows: tiles only where they win clearly.
+    return tile_us * (ratio > 1.0 ? 1.3 : 1.0) < voxel_us;
+}
+
+template <typename T>
+void resample(int mode, int comps, const int (&from)[3], const int (&to)[3], const void *in, void *out,
+              cudaStream_t s) {
+    const T *i = static_cast<const T *>(in);
+    T *o = static_cast<T *>(out);
+    if (tiles_serve(mode, comps, from, to))
+        k_resample<T><<<(int) resample_tiles(to), RS_X * RS_Y, 0, s>>>(i, o, from[0], from[1], from[2], to[0], to[1],
+                                                                      to[2], comps, mode);
+    else
+        k_resample_voxel<T><<<grid_for((long long) to[0] * to[1] * to[2] * comps), 256, 0, s>>>(
+            i, o, from[0], from[1], from[2], to[0], to[1], to[2], comps, mode);
+}
+
 bool dims_ok(size_t nx, size_t ny, size_t nz) {
     return nx >= 1 && ny >= 1 && nz >= 1 && nx < (1u << 30) && ny < (1u << 30) && nz < (1u << 30);
 }
@@ -564,19 +664,11 @@ extern "C" int dtb_resample_device(int precision, int mode, int comps, size_t nx
         return DTB_ERR_ARGUMENT;
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const long long blocks = ((long long) nx2 + RS_X - 1) / RS_X * (((long long) ny2 + RS_Y - 1) / RS_Y) *
-                             (((long long) nz2 + RS_Z - 1) / RS_Z);
-    if (blocks > INT_MAX) {
-        report(__LINE__, __func__, "output too large");
-        return DTB_ERR_ARGUMENT;
-    }
-    const int grid = (int) blocks;
+    const int from[3] = {(int) nx, (int) ny, (int) nz}, to[3] = {(int) nx2, (int) ny2, (int) nz2};
     if (precision == DTB_PRECISION_FP64)
-        k_resample<double><<<grid, 256, 0, s>>>(static_cast<const double *>(in), static_cast<double *>(out), (int) nx,
-                                               (int) ny, (int) nz, (int) nx2, (int) ny2, (int) nz2, comps, mode);
+        resample<double>(mode, comps, from, to, in, out, s);
     else if (precision == DTB_PRECISION_MIXED)
-        k_resample<float><<<grid, 256, 0, s>>>(static_cast<const float *>(in), static_cast<float *>(out), (int) nx,
-                                              (int) ny, (int) nz, (int) nx2, (int) ny2, (int) nz2, comps, mode);
+        resample<float>(mode, comps, from, to, in, out, s);
     else {
         report(__LINE__, __func__, "invalid precision");
         return DTB_ERR_ARGUMENT;

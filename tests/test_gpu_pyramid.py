@@ -132,3 +132,31 @@ def test_driver_matching_matches_reference():
     dev = D.displacement(torch.from_numpy(d["Jt"]).cuda(), mask=torch.from_numpy(d["mask"]).cuda(), **kw)
     assert dev.dtype == torch.float64
     np.testing.assert_array_equal(dev.cpu().numpy(), got)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nearest", [False, True])
+@pytest.mark.parametrize("src,dst,tiles", [
+    ((20, 20, 20), (10, 10, 10), False),
+    ((16, 16, 16), (32, 32, 32), False),
+    ((48, 48, 48), (96, 96, 96), True),
+    ((2000, 1, 2), (4000, 2, 3), False),
+    ((200, 200, 2), (400, 400, 3), False),
+    ((128, 128, 128), (48, 49, 47), False),
+    ((100, 101, 99), (200, 203, 197), True),
+])
+def test_resample_by_tiles_or_by_voxels(dtype, nearest, src, dst, tiles):
+    """Small, narrow and coarser outputs take a thread per voxel, which is up to
+    seven times as fast there; large finer ones take tiles.  The bits are the
+    oracle's either way."""
+    from torch.profiler import ProfilerActivity, profile
+    v = np.random.default_rng(3).standard_normal((3,) + src).astype(dtype)
+    vd = torch.from_numpy(v).cuda()
+    D.resample(vd, dst, nearest)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        got = D.resample(vd, dst, nearest)
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in prof.key_averages())
+    assert ("k_resample_voxel" in names) == (not tiles)
+    np.testing.assert_array_equal(got.cpu().numpy(), P.resample(v, dst, nearest))
