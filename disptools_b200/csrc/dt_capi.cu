@@ -1483,14 +1483,20 @@ int jacobian_device_impl(const Geom &g, const T *field, T *J, cudaStream_t s) {
 }
 
 // Whether the adjoint streams its weights by TMA (k_gather_tma) or reads them
-// by plain loads (k_adjoint_gather): a TMA tile is 32 voxels wide, and rows of
-// a third of that and fewer leave too many of its threads idle.  Adjoint by TMA
+// by plain loads (k_adjoint_gather): a TMA tile is 32 x 16 voxels wide and high,
+// and volumes that leave most of it idle take the plain loads.  Adjoint by TMA
 // and plain, us: FP32 32^3 17 and 19, 64^3 19 and 26, 101 x 97 x 99 46 and 56,
 // 160^3 97 and 159, 181 x 217 x 181 189 and 247; FP64 32^3 17 and 21, 101 x 97
 // x 99 73 and 77, 160^3 194 and 243, 181 x 217 x 181 335 and 372; 200 x 200 x
 // 17 FP32 46 and 56, FP64 65 and 71; 200 x 200 x 11 46 and 48, 64 and 60;
-// 200 x 200 x 8 38 and 38, 65 and 54.
-bool adjoint_streams_weights(const Geom &g) { return g.order == 4 && g.nx >= 12; }
+// 200 x 200 x 8 38 and 38, 65 and 54; low volumes 577 x 3 x 577 64 and 50, 123
+// and 76; 447 x 5 x 447 47 and 52, 82 and 80; 5000 x 20 x 13 72 and 92, 168 and
+// 132; 277 x 277 x 13 53 and 71, 104 and 103.
+template <typename T>
+bool adjoint_streams_weights(const Geom &g) {
+    const double used = (double) g.nx * g.ny / ((double) ((g.nx + 31) / 32 * 32) * ((g.ny + TT_Y - 1) / TT_Y * TT_Y));
+    return g.order == 4 && g.nx >= 12 && used >= (sizeof(T) == 8 ? 0.3 : 0.2);
+}
 
 // The adjoint's path: the weight pass and gather by default, the fused TMA
 // kernel (order 4, a 16-byte-aligned field whose rows are a multiple of 16
@@ -1526,7 +1532,7 @@ int adjoint_device_impl(const Geom &g, const T *field, const T *gJ, T *gout, cud
     gw.ys = (g.nx + v - 1) / v * v;
     gw.zs = gw.ys * g.ny;
     gw.cs = gw.zs * g.nz;
-    bool streams = adjoint_streams_weights(g);
+    bool streams = adjoint_streams_weights<T>(g);
     long long wn = 0;
     char *base = nullptr;
     auto take = [&](const Geom &w) -> int {

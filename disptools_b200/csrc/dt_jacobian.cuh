@@ -317,6 +317,23 @@ cudaError_t launch_jacobian_any(const T *field, const Geom &g, T *J, int num_sms
     return launch_jacobian_async<T, T, JAC_MAP>(field, g, o, num_sms, s);
 }
 
+// Whether the adjoint's weights are faster with a thread per voxel than by
+// tiles: where most of a tile lies outside the volume, and for small volumes of
+// second order, whose neighbours the cache serves as well.  Adjoint by voxels and
+// by tiles, us: FP32, order 4 577 x 577 x 3 53 and 72, 100000 x 3 x 3 54 and 171,
+// 925 x 925 x 7 421 and 302; FP64 577 x 577 x 9 220 and 248, 707 x 707 x 12 433
+// and 418, 594 x 594 x 17 437 and 428; order 2, FP32 40^3 13 and 15, 70^3 24 and
+// 29, 90^3 41 and 41, 110^3 75 and 64, 174 x 174 x 33 57 and 63; FP64 40^3 15 and
+// 19, 81^3 41 and 43, 90^3 56 and 49.
+template <typename T>
+bool voxel_weights_pay(const Geom &g) {
+    const bool narrow = g.nx <= JA_NARROW;
+    const int tx = narrow ? JaTile<8>::X : JaTile<32>::X, ty = narrow ? JaTile<8>::Y : JaTile<32>::Y;
+    const double used = (double) g.nx * g.ny / ((double) ((g.nx + tx - 1) / tx * tx) * ((g.ny + ty - 1) / ty * ty));
+    if (used < (sizeof(T) == 8 && narrow ? 0.7 : 0.4)) return true;
+    return g.order == 2 && used * g.nx * g.ny * g.nz < (sizeof(T) == 8 ? 5.5e5 : 7e5);
+}
+
 template <typename T>
 cudaError_t launch_weights_any(const T *field, const Geom &g, const T *gJ, T *W, long long wn, long long wys,
                                long long wzs, int num_sms, cudaStream_t s) {
@@ -326,6 +343,7 @@ cudaError_t launch_weights_any(const T *field, const Geom &g, const T *gJ, T *W,
     o.wn = wn;
     o.wys = wys;
     o.wzs = wzs;
+    if (voxel_weights_pay<T>(g)) return launch_weights_voxel<T>(field, g, gJ, W, wn, wys, wzs, s);
     return launch_jacobian_async<T, T, JAC_WEIGHTS>(field, g, o, num_sms, s);
 }
 

@@ -338,12 +338,61 @@ __device__ __forceinline__ int ldcg_int(const int *p) { return __ldcg(p); }
 
 // ------------------------------------------------------------------------
 // Exact adjoint of the Jacobian stencil (for autograd).
-// Pass 1 (k_jacobian_tma or k_jacobian_async): W[c][a](p) = w(p) *
+// Pass 1 (k_jacobian_tma, k_jacobian_async or k_adjoint_w): W[c][a](p) = w(p) *
 // cof_ca(I + A(p)) * ih_a, A the stencil matrix.
 // Pass 2: grad_c(q) = sum_a sum_t W[c][a](q - t e_a) * kappa(k_a(q - t e_a), t).
 // W is dense, [9][nz][ny][nx] with component stride wn.  Where the caller
 // prefers this gather to k_gather_tma: adjoint_streams_weights in dt_capi.cu.
 // ------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ T gload_deriv(const T *f, long long o, long long s, int k, T ih) {
+    switch (k) {
+    case S_FWD: return fd_fwd<T>(f[o], f[o + s], f[o + 2 * s], ih);
+    case S_BWD: return fd_bwd<T>(f[o], f[o - s], f[o - 2 * s], ih);
+    case S_C2: return fd_c2<T>(f[o + s], f[o - s], ih);
+    default: return fd_c4<T>(f[o + s], f[o - s], f[o + 2 * s], f[o - 2 * s], ih);
+    }
+}
+
+// The weights with a thread per voxel, its neighbours by plain loads: for the
+// volumes that launch_weights_any sends here.  Bound by the loads in flight: at
+// 48 registers in FP32, five blocks an SM, the adjoint of 1414 x 1414 x 3 takes
+// 340 us, at 40 and six 309.
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4)
+    k_adjoint_w(Geom g, const T *__restrict__ f, const T *__restrict__ gJ, T *__restrict__ W, long long wn,
+                long long wys, long long wzs) {
+    const long long N = (long long) g.nx * g.ny * g.nz;
+    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < N;
+         i += (long long) gridDim.x * blockDim.x) {
+        const int x = (int) (i % g.nx);
+        const int y = (int) ((i / g.nx) % g.ny);
+        const int z = (int) (i / ((long long) g.nx * g.ny));
+        int k[3];
+        schemes_at(x, y, z, g, k);
+        const long long o = (long long) z * g.zs + (long long) y * g.ys + x;
+        const long long st[3] = {1, g.ys, g.zs};
+        T m[3][3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) m[c][a] = gload_deriv<T>(f + c * g.cs, o, st[a], k[a], (T) g.ih[a]) + (c == a ? T(1) : T(0));
+        const T w = gJ[o];
+        T *out = W + (z * wzs + y * wys + x);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int r0 = c == 0 ? 1 : 0, r1 = c == 2 ? 1 : 2;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const int c0 = a == 0 ? 1 : 0, c1 = a == 2 ? 1 : 2;
+                const T minor = m[r0][c0] * m[r1][c1] - m[r0][c1] * m[r1][c0];
+                const T cof = ((c + a) & 1) ? -minor : minor;
+                out[(c * 3 + a) * wn] = w * cof * (T) g.ih[a];
+            }
+        }
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ T kappa(int k, int t) {
     switch (k) {
@@ -475,6 +524,15 @@ __global__ void k_regularise(T *__restrict__ J, long long n, T eps) {
 inline int elementwise_grid(long long n) {
     long long b = (n + 255) / 256;
     return (int) (b < 148 * 16 ? (b < 1 ? 1 : b) : 148 * 16);
+}
+
+template <typename T>
+cudaError_t launch_weights_voxel(const T *field, const Geom &g, const T *gJ, T *W, long long wn, long long wys,
+                                 long long wzs, cudaStream_t s) {
+    const long long N = (long long) g.nx * g.ny * g.nz;
+    k_adjoint_w<T><<<elementwise_grid(N), 256, 0, s>>>(g, field, gJ, W, wn, wys, wzs);
+    count_launch();
+    return cudaGetLastError();
 }
 
 template <typename T>

@@ -15,3 +15,21 @@ def ball_problem(n: int = 40, centre: float = 20.0, radius: float = 10.0, inside
 def masked_max(J, Jt, mask) -> float:
     d = np.abs(J - Jt)[mask]
     return float(d.max()) if d.size else 0.0
+
+
+def kernels_of(call):
+    """The call's result and the names of the kernels it ran.  The profiler can
+    lose the records of the first launches, so it sees several calls."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            for _ in range(4):
+                out = call()
+                torch.cuda.synchronize()
+        names = " ".join(e.key for e in prof.key_averages())
+        if "k_" in names:
+            break
+    return out, names

@@ -149,14 +149,9 @@ def test_resample_by_tiles_or_by_voxels(dtype, nearest, src, dst, tiles):
     """Small, narrow and coarser outputs take a thread per voxel, which is up to
     seven times as fast there; large finer ones take tiles.  The bits are the
     oracle's either way."""
-    from torch.profiler import ProfilerActivity, profile
+    from tests.helpers import kernels_of
     v = np.random.default_rng(3).standard_normal((3,) + src).astype(dtype)
     vd = torch.from_numpy(v).cuda()
-    D.resample(vd, dst, nearest)
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        got = D.resample(vd, dst, nearest)
-        torch.cuda.synchronize()
-    names = " ".join(e.key for e in prof.key_averages())
+    got, names = kernels_of(lambda: D.resample(vd, dst, nearest))
     assert ("k_resample_voxel" in names) == (not tiles)
     np.testing.assert_array_equal(got.cpu().numpy(), P.resample(v, dst, nearest))

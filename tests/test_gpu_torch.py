@@ -347,3 +347,35 @@ def test_backward_on_a_thread_without_a_context():
             "torch.autograd.grad(J, f, w)\n"
             "torch.cuda.synchronize()\n")
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
+
+
+@pytest.mark.parametrize("shape, order, weights, gather", [
+    ((6, 18, 33), 2, "k_adjoint_w", "k_adjoint_gather"),
+    ((130, 97, 99), 2, "k_jacobian_async", "k_adjoint_gather"),
+    ((300, 3, 3), 4, "k_adjoint_w", "k_adjoint_gather"),
+    ((40, 41, 3), 4, "k_adjoint_w", "k_adjoint_gather"),
+    ((30, 3, 71), 4, "k_adjoint_w", "k_adjoint_gather"),
+    ((50, 16, 63), 4, "k_jacobian_async", "k_gather_tma"),
+    ((20, 64, 7), 4, "k_jacobian_async", "k_adjoint_gather"),
+])
+def test_adjoint_by_tiles_or_by_voxels(oracle, oracle_pd2, shape, order, weights, gather):
+    """Small volumes of second order and those that leave a tile mostly idle
+    take their weights with a thread per voxel (up to three times as fast
+    there), low ones their gather by plain loads; the identity and tolerances of
+    test_adjoint_of_odd_widths hold for each."""
+    import torch
+    from disptools_b200 import torch_ops
+    from tests.helpers import kernels_of
+    rng = np.random.default_rng(sum(shape) + order)
+    u, v = rng.normal(scale=0.2, size=(2, 3) + shape)
+    w = rng.standard_normal(shape)
+    sp = (0.9, 1.1, 1.3)
+    o = oracle if order == 4 else oracle_pd2
+    h = 1e-4
+    dJ = (o.jacobian(u + h * v, sp) - o.jacobian(u - h * v, sp)) / (2 * h)
+    scale = np.sum(np.abs(w * dJ))
+    for dtype, tol in ((torch.float64, 1e-7), (torch.float32, 1e-5)):
+        ud, wd = torch.from_numpy(u).to(dtype).cuda(), torch.from_numpy(w).to(dtype).cuda()
+        g, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(ud, wd, sp, order))
+        assert weights in names and gather in names
+        assert abs(np.sum(g.double().cpu().numpy() * v) - np.sum(w * dJ)) <= tol * scale
