@@ -483,7 +483,8 @@ int dtb_get_trial_kernel(void);
 /* Frees the device memory the library keeps on the current device between
  * calls: the solver's workspace (pitched field buffers, descriptors, tile
  * partials) and the staging area of host-array calls, both of which grow to
- * the largest solve seen and are otherwise kept until the process exits.  No
+ * the largest solve seen, the adjoint's weights, and 2 MiB for small maps of
+ * host arrays; all are otherwise kept until the process exits.  No
  * counterpart in the reference, whose CUDA path allocates and frees its
  * buffers in every call (cuda/displacement_field_gradient.cu:213-236,
  * 458-467).  Returns DTB_OK; must not overlap a running call on the device. */

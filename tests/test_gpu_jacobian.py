@@ -176,3 +176,22 @@ def test_tma_kernel_keeps_infinities_local(oracle, at):
     np.testing.assert_array_equal(np.isfinite(J), np.isfinite(ref))
     ok = np.isfinite(ref)
     assert np.max(np.abs(J[ok] - ref[ok])) <= 2e-5
+
+
+def test_maps_of_host_arrays_on_kept_and_own_memory(oracle):
+    """Maps on both sides of the 2 MiB that are kept (40^3 and 41^3), from
+    threads at once, of which one has them, and after a release."""
+    from concurrent.futures import ThreadPoolExecutor
+    rng = np.random.default_rng(2)
+    fields = [rng.normal(scale=0.2, size=(3, n, n, n)) for n in (8, 31, 32, 33, 40, 41)]
+    refs = [oracle.jacobian(f) for f in fields]
+    dt.release_device_memory()
+    with ThreadPoolExecutor(4) as pool:
+        for _ in range(3):
+            for got, ref in zip(pool.map(dt.jacobian, fields * 3), refs * 3):
+                np.testing.assert_allclose(got, ref, rtol=0, atol=1e-13)
+            for got, ref in zip(pool.map(lambda J: dt.regularise(J, 0.9), refs * 3), refs * 3):
+                np.testing.assert_array_equal(got, np.where(ref < 0.9, 0.9, ref))
+    dt.release_device_memory()
+    for f, ref in zip(fields, refs):
+        np.testing.assert_allclose(dt.jacobian(f), ref, rtol=0, atol=1e-13)
