@@ -379,3 +379,65 @@ def test_adjoint_by_tiles_or_by_voxels(oracle, oracle_pd2, shape, order, weights
         g, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(ud, wd, sp, order))
         assert weights in names and gather in names
         assert abs(np.sum(g.double().cpu().numpy() * v) - np.sum(w * dJ)) <= tol * scale
+
+
+def _off_by_one_element(t):
+    import torch
+    view = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape)
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.parametrize("dtype, shape", [("float64", (193, 197, 198)), ("float32", (37, 39, 68))])
+def test_tma_and_element_wise_stencils_agree(dtype, shape):
+    """Map and weights by the TMA kernel and, for a field off a 16-byte
+    boundary, by the element-wise one, on a size that takes both and has
+    partial tiles along every axis.  FP64 rounds alike; FP32 sums a derivative's
+    two terms, four products a minor and three a determinant in other orders."""
+    import torch
+    from disptools_b200 import torch_ops
+    from tests.helpers import kernels_of
+    tdt = getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    f = 0.1 * torch.randn((3,) + shape, dtype=tdt, device="cuda", generator=g)
+    w = torch.randn(shape, dtype=tdt, device="cuda", generator=g)
+    off = _off_by_one_element(f)
+    sp = (0.9, 1.2, 1.05)
+    for call in (lambda u: torch_ops.jacobian_raw(u, sp), lambda u: torch_ops.jacobian_adjoint_raw(u, w, sp)):
+        tma, names = kernels_of(lambda: call(f))
+        assert "k_jacobian_tma" in names and "k_jacobian_async" not in names
+        plain, names = kernels_of(lambda: call(off))
+        assert "k_jacobian_async" in names and "k_jacobian_tma" not in names
+        if dtype == "float64":
+            torch.testing.assert_close(tma, plain, rtol=0, atol=0)
+        else:
+            torch.testing.assert_close(tma, plain, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("shape", [(20, 21, 45), (5, 31, 13), (9, 16, 67), (35, 17, 99)])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_streamed_and_plain_gathers_agree(dtype, shape):
+    """The gather by TMA and, where a memory limit has no room for padded rows,
+    by plain loads, from the same weights: equal in FP64, and in FP32 thirteen
+    terms a component, each rounded once in either order."""
+    import torch
+    from disptools_b200 import _native as N
+    from disptools_b200 import torch_ops
+    from tests.helpers import kernels_of
+    tdt = getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    f = 0.2 * torch.randn((3,) + shape, dtype=tdt, device="cuda", generator=g)
+    w = torch.randn(shape, dtype=tdt, device="cuda", generator=g)
+    streamed, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(f, w))
+    assert "k_gather_tma" in names and "k_adjoint_gather" not in names
+    n = int(np.prod(shape))
+    try:
+        N.check(N.lib.dtb_set_device_memory_limit(9 * ((n + 63) // 64 * 64) * f.element_size() + 256))
+        plain, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(f, w))
+    finally:
+        N.check(N.lib.dtb_set_device_memory_limit(0))
+    assert "k_adjoint_gather" in names and "k_gather_tma" not in names
+    if dtype == "float64":
+        torch.testing.assert_close(streamed, plain, rtol=0, atol=0)
+    else:
+        assert float((streamed - plain).abs().max()) <= 13 * 2 ** -24 * 13 * float(plain.abs().max())
