@@ -1514,12 +1514,15 @@ extern "C" void generate_displacement_greedy_cuda(
 // ---------------------------------------------------------------------------
 namespace {
 
-// FP64 volumes below this many voxels take the element-wise Jacobian kernel
-// and the plain-load gather whatever their layout.  The TMA kernels run one
-// block of 8 warps per SM in FP64, the element-wise one 16 warps: map of
-// 128^3 63.8 us by TMA, 55.9 element-wise (129 x 127 x 125); 180 x 216 x 180
-// 139 and 132; 192 x 224 x 192 148 and 149.  Adjoint of 160^3 391 us by TMA and
-// 272 without, 180 x 216 x 180 434 and 412, 192 x 224 x 192 454 and 493.
+// FP64 maps and weights of volumes below this many voxels take the element-wise
+// Jacobian kernel whatever their layout.  The TMA kernel runs one block of 8
+// warps per SM in FP64, the element-wise one 16 warps; on wide volumes the two
+// are within 6 % of each other, on volumes at most 16 wide, or low ones, the
+// element-wise kernel is up to 2.7 times as fast.  Map by TMA and element-wise,
+// us: 64^3 8.5 and 10.5, 128^3 37 and 40, 160^3 69.5 and 68, 300 x 300 x 60 95 and
+// 94, 192 x 224 x 192 111 and 117, 198 x 197 x 193 122 and 117, 256^3 218 and 221.
+// Adjoint: 128^3 104 and 105, 192 x 224 x 192 338 and 343, 256^3 694 and 721; 612 x
+// 612 x 16 493 and 433, 707 x 707 x 6 431 and 239, 1224 x 1224 x 4 1098 and 414.
 constexpr long long FP64_ELEMENTWISE_VOXELS = 7500000;
 
 template <typename T>

@@ -2,8 +2,9 @@
 // adjoint's weights, or the log of the map added to a running sum.
 //
 // The TMA kernels need rows a multiple of 16 bytes long.  Every other layout
-// (odd widths, a base off a 16-byte boundary), second order, and FP64
-// arithmetic on float fields come here.
+// (odd widths, a base off a 16-byte boundary), second order, FP64 arithmetic on
+// float fields, and FP64 volumes of less than 7.5 million voxels
+// (FP64_ELEMENTWISE_VOXELS) come here.
 //
 // A block of 32 x 8 threads, one voxel each, marches a 32 x 8 tile through
 // bz planes.  Boxes of the tile with two voxels of halo on each x-y side and
@@ -16,9 +17,9 @@
 //
 // What bounds it: instruction issue and the latency of a plane's chain, so
 // resident warps: one voxel a thread keeps FP32 at 64 registers (four blocks,
-// 32 warps an SM).  Measured against the plain-load kernel it replaced
-// (256 threads, a 64-bit index per load, scheme by case analysis): see the
-// launch wrapper.
+// 32 warps an SM).  Map of 181 x 217 x 181 in FP32 77 us, FP64 108-113 us; the
+// plain-load kernel before it (256 threads, a 64-bit index per load, scheme by
+// case analysis, a lock and a wait) 230 and 330.
 #pragma once
 
 #include <algorithm>

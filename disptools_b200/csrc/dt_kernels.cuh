@@ -4,12 +4,13 @@
 // allowed) and dt_kernels_f64.cu (FP64; compiled with -fmad=false so the
 // per-voxel arithmetic rounds exactly like the reference C library).
 //
-// Every kernel is a 2.5-D stencil: a block of BX x BY threads owns one x-y
-// tile and marches a range of z planes, keeping a ring of planes (with an
-// x-y halo) in shared memory.  Reductions are FP64 whatever the element type:
-// each tile writes one partial, and the last tile of a volume to finish (an
-// atomic ticket, no spinning) folds the partials in a fixed order and runs
-// that volume's step control.  The result is deterministic run to run.
+// Here: the difference schemes and the determinant, the solver's reductions and
+// step control, the adjoint's kernels by plain loads, and element-wise kernels.
+// The tiled stencils that march through z are in dt_kernels_tma.cuh and
+// dt_jacobian.cuh.  Reductions are FP64 whatever the element type: each tile
+// writes one partial, and the last tile of a volume to finish (an atomic ticket,
+// no spinning) folds the partials in a fixed order and runs that volume's step
+// control.  The result is deterministic run to run.
 #pragma once
 
 #include <cfloat>

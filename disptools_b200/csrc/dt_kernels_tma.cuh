@@ -2328,8 +2328,8 @@ cudaError_t launch_jacobian_tma(const CUtensorMap &tm_u, const Geom &g, T *jout,
 // k_gather_tma: the gather pass of the adjoint,
 //   grad_c(q) = sum_a sum_t W[c][a](q - t e_a) * kappa(k_a(q - t e_a), t)
 // (the same taps, coefficients and summation order as k_adjoint_gather), on
-// weights streamed by TMA.  W is [c][a][wn] with the field's row and plane
-// strides.  A 32 x TT_Y tile marches through its z range; the stage of plane
+// weights streamed by TMA.  W is [c][a][wn], its rows padded to 16 bytes where
+// the field's are not.  A 32 x TT_Y tile marches through its z range; the stage of plane
 // q holds W[.][z] of the tile at plane q and, for the gradient plane
 // ze = q - 2, W[.][x] of the tile's rows with four columns each side and
 // W[.][y] of its columns with two rows each side.  Each thread keeps its

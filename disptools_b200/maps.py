@@ -27,9 +27,10 @@ import torch
 from . import _native as N
 from . import io as fio
 
-# Clamp modes of dtb_log_jacobian_accumulate_device
+# Clamp modes of dtb_log_jacobian_accumulate_device (maps of fields are clamped by
+# dtb_log_jacobian_field_device)
 CLAMP_THRESHOLD = 0   # values outside [epsilon, 1e9] become epsilon
-CLAMP_REGULARISE = 1  # values below epsilon become epsilon (fields: dtb_log_jacobian_field_device)
+CLAMP_REGULARISE = 1  # values below epsilon become epsilon
 
 
 def _stream(t: torch.Tensor) -> int:

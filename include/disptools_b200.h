@@ -364,10 +364,11 @@ enum {
 int dtb_volume_change_device(int precision, size_t n, double epsilon, const void *J, void *out,
                              void *stream);
 
-/* acc[i] += log(clamp(J[i])) over n values, acc in FP64: one map of the
- * geometric means of average_jacobian (mode DTB_CLAMP_THRESHOLD,
- * disptools/displacements.py:571-625) and
- * average_jacobian_from_displacements (DTB_CLAMP_REGULARISE, :486-568). */
+/* acc[i] += log(clamp(J[i])) over n values, acc in FP64: one map of a geometric
+ * mean, clamped as average_jacobian (mode DTB_CLAMP_THRESHOLD,
+ * disptools/displacements.py:571-625) or average_jacobian_from_displacements
+ * (DTB_CLAMP_REGULARISE, :486-568) clamps it.  For fields,
+ * dtb_log_jacobian_field_device does this and their maps in one pass. */
 int dtb_log_jacobian_accumulate_device(int precision, int mode, size_t n, double epsilon,
                                        const void *J, double *acc, void *stream);
 

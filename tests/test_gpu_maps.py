@@ -101,3 +101,21 @@ def test_regularise_matches_reference_with_nan():
     from oracle.oracle import Reference
     if Reference.available("ref64"):
         np.testing.assert_array_equal(got, Reference("ref64").regularise(g["regularise_in"], 0.05))
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_log_accumulate_clamped_as_regularise(dtype):
+    """The accumulating entry point with the clamp of
+    average_jacobian_from_displacements (no upper bound, a NaN stays)."""
+    from disptools_b200 import _native as N
+    maps = [torch.from_numpy(J).to(dtype).cuda() for J in _maps(3, seed=4)]
+    maps[1].view(-1)[7] = float("nan")
+    acc = torch.zeros(maps[0].shape, dtype=torch.float64, device="cuda")
+    want = np.zeros(acc.shape)
+    for J in maps:
+        N.check(N.lib.dtb_log_jacobian_accumulate_device(M._prec(J), M.CLAMP_REGULARISE, J.numel(), 1e-5, J.data_ptr(),
+                                                         acc.data_ptr(), M._stream(J)))
+        j = J.double().cpu().numpy()
+        want += np.log(np.where(j < 1e-5, 1e-5, j))
+    # Logs of at most 22 in magnitude, each and each sum good to a few units in the last place.
+    np.testing.assert_allclose(acc.cpu().numpy(), want, rtol=0, atol=1e-13)
