@@ -69,16 +69,19 @@ struct SolverState {
     unsigned int ticket_t;   // block counters of the trial / gradient launches
     unsigned int ticket_g;
     int fault;               // a bounded wait gave up (reported as an error)
+    unsigned long long lost_next;  // address of the next state in TileQueue::lost
     IterLog *log;            // verbose output (null when off)
     long long log_cap, log_n;
 };
 
 // Dynamic tile queue of one persistent launch: blocks take tiles with an
 // atomic counter; the last block to leave resets the queue for the next
-// launch (every block increments `exited` exactly once, after its last take).
+// launch (every block increments `exited` exactly once, after its last take)
+// and ends the volumes that lost a transfer.
 struct TileQueue {
     unsigned int next;
-    unsigned int exited;
+    unsigned int exited;      // blocks that have left; above 2^16: those of them that lost a transfer
+    unsigned long long lost;  // state of a volume that lost a transfer (address), linked by lost_next; 0: none
 };
 
 // Geometry of one volume on the device.

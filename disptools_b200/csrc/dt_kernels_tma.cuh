@@ -118,10 +118,25 @@ struct GradTmaLayout {
     static constexpr int BYTES = BAR_OFF + S * 8;
 };
 
-// Counts a block out of a launch; the last one resets the queue for the next.
-__device__ __forceinline__ void leave_queue(TileQueue *q) {
+// Counts a block out of a launch; the last one resets the queue for the next
+// and ends the volumes that lost a transfer.  Not before: while a launch runs, a
+// volume's state only changes when all its tiles have been worked off, so every
+// thread of every block that takes a tile reads the same (`done` above all: a
+// block whose warps disagreed would part at its barriers).
+__device__ __forceinline__ void leave_queue(TileQueue *q, bool lost = false) {
+    constexpr unsigned LOST = 1u << 16;  // a grid has far fewer blocks
     __threadfence();
-    if (atomicAdd(&q->exited, 1u) == gridDim.x - 1) {
+    const unsigned before = atomicAdd(&q->exited, lost ? 1u + LOST : 1u);
+    if (before % LOST == gridDim.x - 1) {
+        if (lost || before >= LOST) {
+            __threadfence();
+            for (unsigned long long a = __ldcg(&q->lost); a;) {
+                SolverState *st = reinterpret_cast<SolverState *>(a);
+                st->done = 1;
+                a = __ldcg(&st->lost_next);
+            }
+            q->lost = 0;
+        }
         q->next = 0;
         q->exited = 0;
         __threadfence();
@@ -155,14 +170,20 @@ __device__ __forceinline__ unsigned char *align_smem_128(unsigned char *p) {
     return p + ((128u - (a & 127u)) & 127u);
 }
 
-// Records a lost transfer: the volume stops with an error flag that the host
-// reports, and the calling thread waits (bounded) for the transfers of
+// Records a lost transfer: the volume gets an error flag that the host reports
+// and stops with this launch (leave_queue).
+__device__ __forceinline__ void volume_fault(SolverState *st, TileQueue *q) {
+    if (atomicExch(&st->fault, 1)) return;  // listed already
+    st->lost_next = atomicExch(&q->lost, reinterpret_cast<unsigned long long>(st));
+}
+
+// The same, and the calling thread waits (bounded) for the transfers of
 // iterations [from, to) that were issued but not consumed, so none lands in
 // shared memory after the block has left.
 template <int S>
-__device__ __forceinline__ void tma_fault(SolverState *st, uint64_t *bars, uint32_t kbase, int from, int to) {
-    atomicExch(&st->fault, 1);
-    atomicExch(&st->done, 1);
+__device__ __forceinline__ void tma_fault(SolverState *st, TileQueue *q, uint64_t *bars, uint32_t kbase, int from,
+                                          int to) {
+    volume_fault(st, q);
     for (int j = from; j < to; ++j) {
         const uint32_t k = kbase + j;
         mbar_wait_bounded(&bars[k % S], (k / S) & 1u, 1u << 16);
@@ -608,9 +629,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
         const bool stale_zero = GREEDY && (old_b == 0 || !ldcg_int(&st->b0_nonzero));
         const double eta = __ldcg(&st->eta);
         const T tol = (T) st->tolerance, delta = (T) st->delta, zeta = (T) st->zeta;
-        // A block that lost a transfer sets `done` at any time (tma_fault):
-        // the threads agree on what they read, so none goes on alone.
-        if (__syncthreads_or(done)) continue;
+        if (done) continue;  // by every thread alike (leave_queue)
         const bool trial = phase != PH_EVAL0;
         const int lt = tile - V.tile_begin;
         const int txi = lt % V.tiles_x, tyi = (lt / V.tiles_x) % V.tiles_y, tzi = lt / (V.tiles_x * V.tiles_y);
@@ -901,8 +920,8 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
         if (failed) {
             if (GREEDY) cp_async_wait_all();  // no element copy lands after the block has left
             if (tid == 0) {
-                tma_fault<L::S>(st, bars, kbase, fail_it + 1, issued_n);
-                leave_queue(queue);
+                tma_fault<L::S>(st, queue, bars, kbase, fail_it + 1, issued_n);
+                leave_queue(queue, true);
             }
             __syncthreads();
             return;
@@ -997,8 +1016,7 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
         SolverState *st = states + vol;
         const Geom g = V.g;
         const int done = ldcg_int(&st->done), wanted = ldcg_int(&st->need_gradient), old_b = ldcg_int(&st->old_buf);
-        // Agreed on for the whole block, as in the trial kernel.
-        if (__syncthreads_or(done || !wanted)) continue;
+        if (done || !wanted) continue;  // by every thread alike (leave_queue)
         const int lt = tile - V.tile_begin;
         const int txi = lt % V.tiles_x, tyi = (lt / V.tiles_x) % V.tiles_y, tzi = lt / (V.tiles_x * V.tiles_y);
         const int x0 = txi * TXW, y0 = tyi * TT_Y, z0 = tzi * V.bz;
@@ -1312,8 +1330,8 @@ __global__ void __launch_bounds__(TXW / 2 * (TYT + grad_halo_rows<TXW>()), sizeo
         }
         if (failed) {
             if (tid == 0) {
-                tma_fault<L::S>(st, bars, kbase, fail_it + 1, issued_n);
-                leave_queue(queue);
+                tma_fault<L::S>(st, queue, bars, kbase, fail_it + 1, issued_n);
+                leave_queue(queue, true);
             }
             __syncthreads();
             return;
@@ -1731,8 +1749,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
         __syncthreads();  // every warp has left the plane loop
         if (s_fault) {
             if (tid == 0) {
-                atomicExch(&st->fault, 1);
-                atomicExch(&st->done, 1);
+                volume_fault(st, queue);
                 // The last load issued into each slot: wait (bounded) until it
                 // has landed, so nothing arrives after the block has left.
                 const int to = s_issued;
@@ -1740,7 +1757,7 @@ __global__ void __launch_bounds__(TXW / 2 * TYT, (TXW / 2 * TYT <= 256 && sizeof
                     const uint32_t kk = kbase + j;
                     mbar_wait_bounded(&bars[kk % S], (kk / S) & 1u, 1u << 16);
                 }
-                leave_queue(queue);
+                leave_queue(queue, true);
             }
             __syncthreads();
             return;
