@@ -44,7 +44,6 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 #include "dt_internal.h"
 
@@ -687,15 +686,16 @@ struct Slab {
 };
 
 // Pinned copies of the state, two a solve (one per batch of steps in flight).
-// Up to MAX_SPARE are kept for later solves.
+// Up to MAX_SPARE are kept for later solves, in an array: keeping one cannot
+// throw where it goes out of scope.
 struct HostStates {
     MatchState *p = nullptr;
     HostStates() {
         {
-            std::lock_guard<std::mutex> lock(mutex());
-            if (!spare().empty()) {
-                p = spare().back();
-                spare().pop_back();
+            Spare &s = spare();
+            std::lock_guard<std::mutex> lock(s.mutex);
+            if (s.count > 0) {
+                p = s.states[--s.count];
                 return;
             }
         }
@@ -707,9 +707,10 @@ struct HostStates {
     ~HostStates() {
         if (!p) return;
         {
-            std::lock_guard<std::mutex> lock(mutex());
-            if (spare().size() < MAX_SPARE) {
-                spare().push_back(p);
+            Spare &s = spare();
+            std::lock_guard<std::mutex> lock(s.mutex);
+            if (s.count < MAX_SPARE) {
+                s.states[s.count++] = p;
                 return;
             }
         }
@@ -719,14 +720,15 @@ struct HostStates {
     HostStates &operator=(const HostStates &) = delete;
 
 private:
-    static constexpr size_t MAX_SPARE = 8;
-    static std::mutex &mutex() {
-        static std::mutex m;
-        return m;
-    }
-    static std::vector<MatchState *> &spare() {
-        static std::vector<MatchState *> v;
-        return v;
+    static constexpr int MAX_SPARE = 8;
+    struct Spare {
+        std::mutex mutex;
+        MatchState *states[MAX_SPARE] = {};
+        int count = 0;
+    };
+    static Spare &spare() {
+        static Spare s;
+        return s;
     }
 };
 

@@ -217,3 +217,15 @@ def test_matching_of_a_long_column():
     assert float(short.abs().max()) > 0.0
     torch.testing.assert_close(long[:, :300], short[:, :300], rtol=0, atol=1e-5)
     assert not long[:, 300:].any()
+
+
+def test_matching_from_many_threads():
+    """More solves at once than pinned states are kept: each the field of the
+    solve alone."""
+    from concurrent.futures import ThreadPoolExecutor
+    problems = [ball_problem(n, n / 2, n / 4, 1.1) for n in (10, 12, 14, 16)]
+    kw = dict(algorithm="matching", it_max=12)
+    alone = [dt.solve(J, m, **kw)[0] for J, m in problems]
+    with ThreadPoolExecutor(16) as pool:
+        for got, want in zip(pool.map(lambda p: dt.solve(*p, **kw)[0], problems * 8), alone * 8):
+            np.testing.assert_array_equal(got, want)
