@@ -152,6 +152,6 @@ def test_resample_by_tiles_or_by_voxels(dtype, nearest, src, dst, tiles):
     from tests.helpers import kernels_of
     v = np.random.default_rng(3).standard_normal((3,) + src).astype(dtype)
     vd = torch.from_numpy(v).cuda()
-    got, names = kernels_of(lambda: D.resample(vd, dst, nearest))
+    got, names = kernels_of(lambda: D.resample(vd, dst, nearest), "k_resample")
     assert ("k_resample_voxel" in names) == (not tiles)
     np.testing.assert_array_equal(got.cpu().numpy(), P.resample(v, dst, nearest))

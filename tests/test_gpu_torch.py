@@ -376,7 +376,7 @@ def test_adjoint_by_tiles_or_by_voxels(oracle, oracle_pd2, shape, order, weights
     scale = np.sum(np.abs(w * dJ))
     for dtype, tol in ((torch.float64, 1e-7), (torch.float32, 1e-5)):
         ud, wd = torch.from_numpy(u).to(dtype).cuda(), torch.from_numpy(w).to(dtype).cuda()
-        g, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(ud, wd, sp, order))
+        g, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(ud, wd, sp, order), weights, gather)
         assert weights in names and gather in names
         assert abs(np.sum(g.double().cpu().numpy() * v) - np.sum(w * dJ)) <= tol * scale
 
@@ -404,9 +404,9 @@ def test_tma_and_element_wise_stencils_agree(dtype, shape):
     off = _off_by_one_element(f)
     sp = (0.9, 1.2, 1.05)
     for call in (lambda u: torch_ops.jacobian_raw(u, sp), lambda u: torch_ops.jacobian_adjoint_raw(u, w, sp)):
-        tma, names = kernels_of(lambda: call(f))
+        tma, names = kernels_of(lambda: call(f), "k_jacobian_tma")
         assert "k_jacobian_tma" in names and "k_jacobian_async" not in names
-        plain, names = kernels_of(lambda: call(off))
+        plain, names = kernels_of(lambda: call(off), "k_jacobian_async")
         assert "k_jacobian_async" in names and "k_jacobian_tma" not in names
         if dtype == "float64":
             torch.testing.assert_close(tma, plain, rtol=0, atol=0)
@@ -428,12 +428,12 @@ def test_streamed_and_plain_gathers_agree(dtype, shape):
     g = torch.Generator(device="cuda").manual_seed(8)
     f = 0.2 * torch.randn((3,) + shape, dtype=tdt, device="cuda", generator=g)
     w = torch.randn(shape, dtype=tdt, device="cuda", generator=g)
-    streamed, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(f, w))
+    streamed, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(f, w), "k_gather_tma")
     assert "k_gather_tma" in names and "k_adjoint_gather" not in names
     n = int(np.prod(shape))
     try:
         N.check(N.lib.dtb_set_device_memory_limit(9 * ((n + 63) // 64 * 64) * f.element_size() + 256))
-        plain, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(f, w))
+        plain, names = kernels_of(lambda: torch_ops.jacobian_adjoint_raw(f, w), "k_adjoint_gather")
     finally:
         N.check(N.lib.dtb_set_device_memory_limit(0))
     assert "k_adjoint_gather" in names and "k_gather_tma" not in names
